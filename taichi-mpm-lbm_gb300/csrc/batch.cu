@@ -186,13 +186,15 @@ int check_batch(const fsi_batch* b) {
 
 // One CTA per (scene, block of kBlock particles): the single-solver P2G / G2P bodies on the
 // scene's grid block.
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 1024 / kBlock)
     batch_p2g_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
                      const Tile* __restrict__ ptiles, PView P, float4* grid_all, uint8_t* dirty_all) {
+  extern __shared__ float4 scatter_smem[];
+  auto& sm = *reinterpret_cast<ScatterSmem<kBlock>*>(scatter_smem);
   const Tile t = ptiles[blockIdx.x];
   const Mpm m = sol[t.lattice].m;
-  p2g_body(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
-           t.first * kBlock + threadIdx.x);
+  p2g_runs_body<kBlock>(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
+                        t.first * kBlock + threadIdx.x, sm);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -524,7 +526,9 @@ extern "C" int fsi_batch_mpm_substep(const fsi_batch* b, const fsi_particles* pa
   if (b->nptiles == 0) return FSI_OK;
   cudaStream_t s = as_stream(stream);
   float4* g4 = reinterpret_cast<float4*>(grid);
-  batch_p2g_kernel<<<b->nptiles, kBlock, 0, s>>>(b->lat, b->sol, b->ptiles, P, g4, dirty);
+  constexpr size_t smem = sizeof(ScatterSmem<kBlock>);
+  if (int e = opt_in_smem<batch_p2g_kernel>((int)smem)) return e;
+  batch_p2g_kernel<<<b->nptiles, kBlock, smem, s>>>(b->lat, b->sol, b->ptiles, P, g4, dirty);
   if (int e = check_launch("batch_p2g_kernel")) return e;
   batch_g2p_kernel<<<b->nptiles, kBlock, 0, s>>>(b->lat, b->sol, b->ptiles, P, g4);
   if (int e = check_launch("batch_g2p_kernel")) return e;

@@ -88,6 +88,7 @@ template <int kStore, bool kFast>
 __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persistent_kernel(PersistArgs a) {
   extern __shared__ float4 persist_smem[];
   float (*tile)[kTileCap] = reinterpret_cast<float (*)[kTileCap]>(persist_smem);
+  auto& p2g_smem = *reinterpret_cast<ScatterSmem<kBlock>*>(persist_smem);
   unsigned epoch = 0;
   int prev = a.prev;
   int* const words = reinterpret_cast<int*>(a.fa.cnt);  // [count][12] counter words
@@ -136,8 +137,9 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
       for (int ti = blockIdx.x; ti < a.nptiles; ti += gridDim.x) {
         const Tile t = a.ptiles[ti];
         const BatchSolid& S = a.sol[t.lattice];
-        p2g_body<false, true>(S.m, a.P, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
-                              t.first * kBlock + threadIdx.x, nullptr, tile);
+        p2g_runs_body<kBlock>(S.m, a.P, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
+                              t.first * kBlock + threadIdx.x, p2g_smem);
+        __syncthreads();  // the records are no longer read
       }
       if (!grid_barrier(a, epoch)) return;
       for (int ti = blockIdx.x; ti < a.nptiles; ti += gridDim.x) {
@@ -182,7 +184,8 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
 // when the launch could not be made (the kernel's own timeout shows in a->err).
 int FSI_BATCH_PERSIST_NAME(const void* args, bool fast, cudaStream_t stream) {
   const PersistArgs& a = *static_cast<const PersistArgs*>(args);
-  const size_t smem = sizeof(float) * 4 * kTileCap;
+  const size_t tile = sizeof(float) * 3 * kTileCap, runs = sizeof(ScatterSmem<kBlock>);
+  const size_t smem = tile > runs ? tile : runs;
   auto launch = [&](auto kernel) -> int {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)

@@ -38,6 +38,19 @@ inline unsigned grid_for(long long n, int block) {
   return (unsigned)(g < 1 ? 1 : g);
 }
 
+// Opts kernel K into `bytes` of dynamic shared memory, once per device.
+template <auto K>
+int opt_in_smem(int bytes) {
+  static bool done[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return check_launch("cudaGetDevice");
+  if (dev >= 0 && dev < 64 && done[dev]) return FSI_OK;
+  if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+    return check_launch("cudaFuncSetAttribute(shared memory)");
+  if (dev >= 0 && dev < 64) done[dev] = true;
+  return FSI_OK;
+}
+
 // D3Q19 velocities in the reference's order (fsi/lbm3d.py:221-239) and opposites (lbm3d.py:171-174).
 __host__ __device__ constexpr int ex(int q) {
   return (q == 1 || q == 7 || q == 9 || q == 11 || q == 13) ? 1

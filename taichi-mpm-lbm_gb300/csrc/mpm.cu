@@ -4,15 +4,13 @@
 // mass) that is all-zero on entry and left all-zero on exit:
 //   1. p2g:   one thread per particle. Deformation update, fixed-corotated
 //             stress (polar rotation by Newton iteration), then the 27-node
-//             quadratic B-spline scatter, unrolled with the per-axis weights and
-//             offsets formed once. A CTA first bounds its particles' stencils; if
-//             the box fits in shared memory the scatter goes to a shared tile (odd
-//             lanes walk the stencil backwards, so the two particles of a sub-cell
-//             pair add into different nodes) and the tile is flushed with one
-//             vector reduction per touched node. Otherwise each particle reduces
-//             straight into global memory. Touched 4^3 node blocks are marked dirty.
-//             The coupled substep forms each particle's penalty force in the same
-//             pass on small launches, or in a separate kernel before it.
+//             quadratic B-spline scatter: a CTA sorts its particles by base cell
+//             in shared memory and sums them in runs, node sums in registers, one
+//             vector reduction into global memory per node a run leaves behind.
+//             Touched 4^3 node blocks are marked dirty. The coupled substep forms
+//             each particle's penalty force in a separate kernel before it, or on
+//             small launches in the same pass, which then scatters through a
+//             shared-memory tile of nodes.
 //   2. g2p:   grid update (p/m + dt g, sticky/damped walls) fused into the
 //             gather: a CTA stages the grid-updated velocities of its stencil box
 //             in shared memory, then each particle gathers v and the APIC C,
@@ -29,16 +27,17 @@
 namespace fsi {
 namespace {
 
-// P2G and G2P are capped at 64 registers (4 CTAs, 32 warps per SM, against 3 CTAs at their
-// natural 75-80): the extra resident warps hide more of the tile-atomic and gather latency
-// (measured: 2,097,152-particle substep 0.475 -> 0.450 ms with P2G capped, 0.454 ms with G2P
-// capped; no spills in P2G, 8 bytes in G2P).
-// Threads per block kT (m.threads): 128, 256 or 512, each at the same 64-register cap.
+// P2G and G2P are capped at 64 registers (32 warps per SM, against 24 at their natural 75-80):
+// the extra resident warps hide more of the gather latency.
+// Threads per P2G / G2P block kT (m.threads): 128, 256 or 512, each at the same 64-register
+// cap; P2G's shared memory is dynamic.
 template <int kT>
 __global__ void __launch_bounds__(kT, 1024 / kT) p2g_kernel(Mpm m, PView P,
                                                             float4* __restrict__ grid,
                                                             uint8_t* __restrict__ dirty) {
-  p2g_body(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x);
+  extern __shared__ float4 scatter_smem[];
+  p2g_runs_body<kT>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x,
+                    *reinterpret_cast<ScatterSmem<kT>*>(scatter_smem));
 }
 
 // The penalty coupling alone (one thread per particle), before p2g_kernel on large launches.
@@ -62,7 +61,7 @@ __global__ void __launch_bounds__(kBlock) coupling_spread_kernel(ForceArgs fa) {
 template <int kT>
 __global__ void __launch_bounds__(kT) coupled_p2g_kernel(Mpm m, PView P, float4* __restrict__ grid,
                                                          uint8_t* __restrict__ dirty, ForceArgs fa) {
-  p2g_body<true>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x, &fa);
+  coupled_p2g_tile_body(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x, fa);
 }
 
 template <int kT>
@@ -71,33 +70,38 @@ __global__ void __launch_bounds__(kT, 1024 / kT) g2p_kernel(Mpm m, PView P,
   g2p_body(m, P, grid, blockIdx.x * kT + threadIdx.x);
 }
 
-// Launches K<m.threads> over the particles.
+// Launches K<threads> over the particles.
 template <template <int> class K, class... Args>
-int launch_tiled(const Mpm& m, cudaStream_t s, const char* what, Args... args) {
-  switch (m.threads) {
-    case 128: K<128>::run(grid_for(m.n, 128), s, args...); break;
-    case 512: K<512>::run(grid_for(m.n, 512), s, args...); break;
-    default: K<256>::run(grid_for(m.n, 256), s, args...); break;
+int launch_tiled(int threads, const Mpm& m, cudaStream_t s, const char* what, Args... args) {
+  switch (threads) {
+    case 128: return K<128>::run(grid_for(m.n, 128), s, what, args...);
+    case 512: return K<512>::run(grid_for(m.n, 512), s, what, args...);
+    default: return K<256>::run(grid_for(m.n, 256), s, what, args...);
   }
-  return check_launch(what);
 }
 template <int kT>
 struct P2G {
-  static void run(unsigned g, cudaStream_t s, Mpm m, PView P, float4* grid, uint8_t* dirty) {
-    p2g_kernel<kT><<<g, kT, 0, s>>>(m, P, grid, dirty);
+  static int run(unsigned g, cudaStream_t s, const char* what, Mpm m, PView P, float4* grid,
+                 uint8_t* dirty) {
+    constexpr size_t b = sizeof(ScatterSmem<kT>);
+    if (int e = opt_in_smem<p2g_kernel<kT>>((int)b)) return e;
+    p2g_kernel<kT><<<g, kT, b, s>>>(m, P, grid, dirty);
+    return check_launch(what);
   }
 };
 template <int kT>
 struct CoupledP2G {
-  static void run(unsigned g, cudaStream_t s, Mpm m, PView P, float4* grid, uint8_t* dirty,
-                  ForceArgs fa) {
+  static int run(unsigned g, cudaStream_t s, const char* what, Mpm m, PView P, float4* grid,
+                 uint8_t* dirty, ForceArgs fa) {
     coupled_p2g_kernel<kT><<<g, kT, 0, s>>>(m, P, grid, dirty, fa);
+    return check_launch(what);
   }
 };
 template <int kT>
 struct G2P {
-  static void run(unsigned g, cudaStream_t s, Mpm m, PView P, const float4* grid) {
+  static int run(unsigned g, cudaStream_t s, const char* what, Mpm m, PView P, const float4* grid) {
     g2p_kernel<kT><<<g, kT, 0, s>>>(m, P, grid);
+    return check_launch(what);
   }
 };
 
@@ -214,8 +218,8 @@ extern "C" int fsi_mpm_substep(const fsi_mpm_desc* d, const fsi_particles* parts
   if (m.n == 0) return FSI_OK;
   cudaStream_t s = as_stream(stream);
   float4* g4 = reinterpret_cast<float4*>(grid);
-  if (int e = launch_tiled<P2G>(m, s, "p2g_kernel", m, P, g4, dirty)) return e;
-  if (int e = launch_tiled<G2P>(m, s, "g2p_kernel", m, P, (const float4*)g4)) return e;
+  if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel", m, P, g4, dirty)) return e;
+  if (int e = launch_tiled<G2P>(m.threads, m, s, "g2p_kernel", m, P, (const float4*)g4)) return e;
   const long long nblocks = (long long)m.nbx * m.nby * m.nbz;
   clear_dirty_kernel<<<grid_for(nblocks, kBlock), kBlock, 0, s>>>(m, g4, dirty);
   return check_launch("clear_dirty_kernel");
@@ -372,8 +376,8 @@ extern "C" int fsi_mpm_substep_noalloc(const fsi_mpm_desc* d, const fsi_particle
   if (cudaMemsetAsync(g4, 0, (size_t)nodes * sizeof(float4), s) != cudaSuccess ||
       cudaMemsetAsync(dirty, 0, (size_t)nblocks, s) != cudaSuccess)
     return check_launch("no-alloc scratch clear");
-  if (int e = launch_tiled<P2G>(m, s, "p2g_kernel (no-alloc)", m, P, g4, dirty)) return e;
-  if (int e = launch_tiled<G2P>(m, s, "g2p_kernel (no-alloc)", m, P, (const float4*)g4)) return e;
+  if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel (no-alloc)", m, P, g4, dirty)) return e;
+  if (int e = launch_tiled<G2P>(m.threads, m, s, "g2p_kernel (no-alloc)", m, P, (const float4*)g4)) return e;
   clear_kernel<<<grid_for(nblocks * 32, kBlock), kBlock, 0, s>>>(m, g4, dirty);
   return check_launch("clear_kernel (no-alloc)");
 }
@@ -416,19 +420,19 @@ extern "C" int fsi_coupled_substep_tiled(const fsi_coupling_desc* c, const fsi_m
   // separate against 3.93 ms fused). m.fold overrides the choice.
   const bool fold = m.fold == 1 || (m.fold == 0 && m.n < 2 * 152 * kBlock);
   if (fold) {
-    if (int e = launch_tiled<CoupledP2G>(m, s, "coupled_p2g_kernel", m, P, g4, dirty, fa)) return e;
+    if (int e = launch_tiled<CoupledP2G>(m.threads, m, s, "coupled_p2g_kernel", m, P, g4, dirty, fa)) return e;
   } else if (m.fold == 3) {
     coupling_gather_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
     if (int e = check_launch("coupling_gather_kernel")) return e;
     coupling_spread_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
     if (int e = check_launch("coupling_spread_kernel")) return e;
-    if (int e = launch_tiled<P2G>(m, s, "p2g_kernel", m, P, g4, dirty)) return e;
+    if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel", m, P, g4, dirty)) return e;
   } else {
     coupling_only_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
     if (int e = check_launch("coupling_only_kernel")) return e;
-    if (int e = launch_tiled<P2G>(m, s, "p2g_kernel", m, P, g4, dirty)) return e;
+    if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel", m, P, g4, dirty)) return e;
   }
-  if (int e = launch_tiled<G2P>(m, s, "g2p_kernel", m, P, (const float4*)g4)) return e;
+  if (int e = launch_tiled<G2P>(m.threads, m, s, "g2p_kernel", m, P, (const float4*)g4)) return e;
   const long long nblocks = (long long)m.nbx * m.nby * m.nbz;
   clear_dirty_kernel<<<grid_for(nblocks, kBlock), kBlock, 0, s>>>(m, g4, dirty);
   return check_launch("clear_dirty_kernel");

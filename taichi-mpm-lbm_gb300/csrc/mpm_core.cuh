@@ -275,19 +275,323 @@ __device__ __forceinline__ void p2g_stress_affine(const Mpm& m, const PView& P, 
   for (int i = 0; i < 9; ++i) affine[i] = __fadd_rn(__fmul_rn(coef, S[i]), __fmul_rn(mass, Cp[i]));
 }
 
-// P2G of particle p (this thread) within its CTA; every thread of the CTA calls it.
-// kCoupled folds _compute_coupling_forces_kernel (fsi/coupling.py:332-406) in front of the
-// scatter: the particle's coupling force is formed first (it is P2G's dt f term) and the
-// fluid reaction and solid fraction are spread into fa.accum beside the grid scatter.
-// kExtTile: the tile is the caller's shared memory `ext` (4 x kTileCap floats) instead of a
-// static array of its own (a kernel that also runs g2p_body then holds one tile, not two).
-template <bool kCoupled = false, bool kExtTile = false>
-__device__ __forceinline__ void p2g_body(const Mpm& m, const PView& P, float4* __restrict__ grid,
-                                         uint8_t* __restrict__ dirty, int p,
-                                         const ForceArgs* fa = nullptr,
-                                         float (*ext)[kTileCap] = nullptr) {
-  __shared__ float own[kExtTile ? 1 : 4][kExtTile ? 1 : kTileCap];
-  float (*tile)[kTileCap] = kExtTile ? ext : reinterpret_cast<float (*)[kTileCap]>(own);
+// Exclusive scan over the block (blockDim.x a multiple of 32, at most 1024 threads).
+// `ws` is 32 ints of shared scratch; *total receives the block's sum.
+__device__ __forceinline__ int block_excl_scan(int v, int* ws, int* total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) ws[wid] = incl;
+  __syncthreads();
+  if (wid == 0) {
+    int s = lane < nw ? ws[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
+    }
+    ws[lane] = s;
+  }
+  __syncthreads();
+  const int excl = incl - v + (wid > 0 ? ws[wid - 1] : 0);
+  *total = ws[nw - 1];
+  __syncthreads();
+  return excl;
+}
+
+// ------------------------------------------------- P2G of a CTA's particles, in runs
+//
+// The scatter sums what a CTA's particles add to a node before anything is added in global
+// memory. Each thread writes its particle's record (weights, affine, momentum) into shared
+// memory at the particle's place in base-cell order: a counting sort over the base cells of the
+// CTA's bounding box, integers only, ties in thread order. The records are then cut into equal
+// runs, one per group of nine lanes: lane (ox, oy) of a group walks its run and keeps the sums
+// of the nodes (ox, oy, 0..2) of the current base cell in registers. A step to the next cell
+// along z retires one node and shifts the other two, any other step retires all three. A
+// retired node is one vector reduction into global memory.
+//
+// Why: particles of a body are stored cell by cell, so 256 of them fill 80 to 120 base cells,
+// and a float atomic in shared memory is a compare-and-swap loop. A tile of nodes in shared
+// memory takes 108 of them per particle (27 nodes, four components); here there are none, and
+// about 5 vector reductions per particle. Measured, one launch for 2,097,152 / 502,304
+// particles: 359 / 115 us with the tile, 188 / 49 us with runs. Adding the runs up once more per
+// node in shared memory, for one reduction per node and CTA, took 340 us: its barriers, and runs
+// cut at the ends of lines.
+constexpr int kScatterCells = 2048;  // base cells of the bounding box that the sort counts
+
+// A particle's record in shared memory, as float offsets: 0-2 wx, 3 mass, 4-6 wy, 7 cell key,
+// 8-10 wz, 11 fz, 12-20 affine, 21-23 m v + dt f, 24-25 fx, fy. 28 floats: 16 bytes short of 128,
+// so records of neighbouring places start on different banks.
+constexpr int kRecFloats = 28;
+
+// Shared memory of the P2G of kT threads (dynamic: 29 KB for 256 threads).
+template <int kT>
+struct __align__(16) ScatterSmem {
+  // the sort's counts, then the records
+  float rec[kT * kRecFloats > kScatterCells ? kT * kRecFloats : kScatterCells];
+  int16_t arrived[kT];
+  int ws[32];
+  int box[8];
+};
+
+// A CTA's particles in base-cell order.
+struct CellOrder {
+  int lo[3];     // lowest base cell
+  int ext[3];    // base cells of the bounding box
+  int count;     // particles
+  int pos;       // this thread's place
+  uint32_t key;  // its cell relative to lo: x, y, z in 10 bits each
+  bool fits;     // the box fits the sort
+};
+
+// `in`: this thread's particle takes part, with base cell `base` in [-2, n) on each axis. Every
+// thread of the CTA calls it; it ends after a barrier that follows the last read of the counts.
+template <int kT>
+__device__ __forceinline__ CellOrder cell_order(bool in, const int base[3], ScatterSmem<kT>& sm) {
+  int* const cnt = reinterpret_cast<int*>(sm.rec);
+  int* const sh = sm.box;
+  CellOrder o;
+  if (threadIdx.x < 3) { sh[threadIdx.x] = 0x7fffffff; sh[3 + threadIdx.x] = -0x7fffffff; }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int lo = __reduce_min_sync(0xffffffffu, in ? base[a] : 0x7fffffff);
+    const int hi = __reduce_max_sync(0xffffffffu, in ? base[a] : -0x7fffffff);
+    if ((threadIdx.x & 31) == 0) { atomicMin(&sh[a], lo); atomicMax(&sh[3 + a], hi); }
+  }
+  o.count = __syncthreads_count(in);
+  o.pos = 0;
+  o.key = 0;
+  long long cells = 1;
+  bool narrow = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    o.lo[a] = sh[a];
+    o.ext[a] = o.count ? sh[3 + a] - sh[a] + 1 : 0;
+    cells *= o.ext[a];
+    narrow = narrow && o.ext[a] < 1023;
+  }
+  o.fits = narrow && cells <= kScatterCells;
+  if (!o.fits || o.count == 0) return o;
+  const int nc = (int)cells;
+  for (int c = threadIdx.x; c < nc; c += kT) cnt[c] = 0;
+  __syncthreads();
+  int cell = 0, slot = 0;
+  if (in) {
+    const int l0 = base[0] - o.lo[0], l1 = base[1] - o.lo[1], l2 = base[2] - o.lo[2];
+    o.key = ((uint32_t)l0 << 20) | ((uint32_t)l1 << 10) | (uint32_t)l2;
+    cell = (l0 * o.ext[1] + l1) * o.ext[2] + l2;
+    slot = atomicAdd(&cnt[cell], 1);
+  }
+  __syncthreads();
+  const int per = (nc + kT - 1) / kT;
+  const int c0 = threadIdx.x * per;
+  int sum = 0;
+  for (int c = c0; c < min(c0 + per, nc); ++c) sum += cnt[c];
+  int total;
+  int run = block_excl_scan(sum, sm.ws, &total);
+  for (int c = c0; c < min(c0 + per, nc); ++c) {
+    const int v = cnt[c];
+    cnt[c] = run;
+    run += v;
+  }
+  __syncthreads();
+  // order of arrival within the cell -> thread order
+  const int start = cnt[cell], end = cell + 1 < nc ? cnt[cell + 1] : o.count;
+  if (in) sm.arrived[start + slot] = (int16_t)threadIdx.x;
+  __syncthreads();
+  if (in) {
+    o.pos = start;
+    for (int s = start; s < end; ++s) o.pos += sm.arrived[s] < (int)threadIdx.x;
+  }
+  return o;
+}
+
+// Adds the records in `rec` (in cell order) into the grid.
+template <int kT>
+__device__ __forceinline__ void scatter_runs(const Mpm& m, const CellOrder& o, const float* rec,
+                                             float4* __restrict__ grid) {
+  constexpr int kGroups = kT / 32 * 3;
+  constexpr uint32_t kNone = 0xfffffff0u;  // no cell: neither it nor the next is a key
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int grp = lane / 9, r9 = lane - 9 * grp;
+  const int ox = r9 / 3, oy = r9 - 3 * ox;
+  const int per = (o.count + kGroups - 1) / kGroups;
+  int q = (warp * 3 + grp) * per;
+  const int end = grp < 3 ? min(q + per, o.count) : q;  // lanes 27-31 have no group
+  const float fox = (float)ox, foy = (float)oy;
+  float am[3][4];
+#pragma unroll
+  for (int z = 0; z < 3; ++z) am[z][0] = am[z][1] = am[z][2] = am[z][3] = 0.f;
+  uint32_t cur = kNone;
+  bool row = false;    // the lane's (x, y) lies in the grid
+  int k0 = 0;          // z of the current base cell
+  long long node = 0;  // index of node (ox, oy, 0) of the current base cell
+  auto retire = [&](int z) {
+    if (row && k0 + z >= 0 && k0 + z < m.nz)
+      red_add_v4(grid + node + z, am[z][0], am[z][1], am[z][2], am[z][3]);
+  };
+  for (; q < end; ++q) {
+    const float* r = rec + q * kRecFloats;
+    const uint32_t key = __float_as_uint(r[7]);
+    if (key != cur) {
+      if (key == cur + 1u) {
+        retire(0);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) { am[0][a] = am[1][a]; am[1][a] = am[2][a]; am[2][a] = 0.f; }
+        ++k0;
+        ++node;
+      } else {
+        if (cur != kNone) {
+          retire(0); retire(1); retire(2);
+#pragma unroll
+          for (int z = 0; z < 3; ++z) am[z][0] = am[z][1] = am[z][2] = am[z][3] = 0.f;
+        }
+        const int i = o.lo[0] + (int)(key >> 20) + ox, j = o.lo[1] + (int)((key >> 10) & 1023u) + oy;
+        k0 = o.lo[2] + (int)(key & 1023u);
+        row = i >= 0 && i < m.nx && j >= 0 && j < m.ny;
+        node = node_index(m, i, j, k0);
+      }
+      cur = key;
+    }
+    const float wxy = __fmul_rn(r[ox], r[4 + oy]);
+    const float4 wz = *reinterpret_cast<const float4*>(r + 8);
+    const float w[3] = {__fmul_rn(wxy, wz.x), __fmul_rn(wxy, wz.y), __fmul_rn(wxy, wz.z)};
+    const float2 f = *reinterpret_cast<const float2*>(r + 24);
+    const float d0 = __fsub_rn(fox, f.x), d1 = __fsub_rn(foy, f.y);
+    const float4 a0 = *reinterpret_cast<const float4*>(r + 12);
+    const float4 a1 = *reinterpret_cast<const float4*>(r + 16);
+    const float4 a2 = *reinterpret_cast<const float4*>(r + 20);
+    const float mass = r[3];
+    // m v + dt f + A (node - x): the terms of ox and oy once for the three oz
+    const float p0 = fmaf(a0.x, d0, fmaf(a0.y, d1, a2.y));
+    const float p1 = fmaf(a0.w, d0, fmaf(a1.x, d1, a2.z));
+    const float p2 = fmaf(a1.z, d0, fmaf(a1.w, d1, a2.w));
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+      const float d2 = __fsub_rn((float)z, wz.w);
+      am[z][0] = fmaf(w[z], fmaf(a0.z, d2, p0), am[z][0]);
+      am[z][1] = fmaf(w[z], fmaf(a1.y, d2, p1), am[z][1]);
+      am[z][2] = fmaf(w[z], fmaf(a2.x, d2, p2), am[z][2]);
+      am[z][3] = fmaf(w[z], mass, am[z][3]);
+    }
+  }
+  if (cur != kNone) { retire(0); retire(1); retire(2); }
+}
+
+// Whether a stencil with this base cell has a node in the grid.
+__device__ __forceinline__ bool stencil_in_grid(int nx, int ny, int nz, const int base[3]) {
+  return base[0] >= -2 && base[0] < nx && base[1] >= -2 && base[1] < ny && base[2] >= -2 &&
+         base[2] < nz;
+}
+
+// Marks the 4^3 node blocks that the stencils of the base cells lo .. lo + ext - 1 overlap.
+__device__ __forceinline__ void mark_cells(const Mpm& m, uint8_t* __restrict__ dirty,
+                                           const int lo[3], const int ext[3]) {
+  const int n[3] = {m.nx, m.ny, m.nz};
+  int b0[3], nb[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    b0[a] = max(lo[a], 0) >> 2;
+    nb[a] = (min(lo[a] + ext[a] + 1, n[a] - 1) >> 2) - b0[a] + 1;
+  }
+  for (int t = threadIdx.x; t < nb[0] * nb[1] * nb[2]; t += blockDim.x) {
+    const int bi = b0[0] + t / (nb[1] * nb[2]), bj = b0[1] + (t / nb[2]) % nb[1], bk = b0[2] + t % nb[2];
+    dirty[((long long)bi * m.nby + bj) * m.nbz + bk] = 1;
+  }
+}
+
+// P2G of particle p (this thread) within its CTA of kT threads, in runs; every thread calls it.
+// A CTA whose bounding box does not fit the sort (particles of two bodies far apart, or
+// scattered ones) adds each contribution straight into global memory.
+template <int kT>
+__device__ __forceinline__ void p2g_runs_body(const Mpm& m, const PView& P, float4* __restrict__ grid,
+                                              uint8_t* __restrict__ dirty, int p,
+                                              ScatterSmem<kT>& sm) {
+  const long long cap = m.cap;
+  const bool act = p < m.n && P.active[p] != 0;
+  int base[3] = {0, 0, 0};
+  float fx[3] = {0.f, 0.f, 0.f};
+  if (act) {
+    float x[3];
+    load_particle_x(P, cap, p, x);
+    base_fx(m, x, base, fx);
+  }
+  const bool in = act && stencil_in_grid(m.nx, m.ny, m.nz, base);
+  const CellOrder o = cell_order(in, base, sm);
+  float affine[9], mv[3], dtf[3], mass = 0.f;
+  if (act) {
+    p2g_stress_affine(m, P, p, affine, mass);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      mv[a] = __fmul_rn(mass, P.v[a * cap + p]);
+      dtf[a] = __fmul_rn(m.dt, P.fp[a * cap + p]);
+    }
+  }
+  if (o.count == 0) return;  // no stencil of this CTA reaches the grid
+  if (o.fits) {
+    if (in) {
+      float* r = sm.rec + o.pos * kRecFloats;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        r[i] = bspline_w(fx[0], i);
+        r[4 + i] = bspline_w(fx[1], i);
+        r[8 + i] = bspline_w(fx[2], i);
+      }
+      r[3] = mass;
+      r[7] = __uint_as_float(o.key);
+      r[11] = fx[2];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) r[12 + i] = __fmul_rn(affine[i], m.dx);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) r[21 + a] = __fadd_rn(mv[a], dtf[a]);
+      r[24] = fx[0];
+      r[25] = fx[1];
+    }
+    __syncthreads();
+    scatter_runs<kT>(m, o, sm.rec, grid);
+    mark_cells(m, dirty, o.lo, o.ext);
+    return;
+  }
+  if (!in) return;
+#pragma unroll 1
+  for (int s = 0; s < 27; ++s) {
+    const int oi = s / 9, oj = (s / 3) % 3, ok = s % 3;
+    const int i = base[0] + oi, j = base[1] + oj, k = base[2] + ok;
+    if (!inside(m, i, j, k)) continue;
+    const float w = __fmul_rn(__fmul_rn(bspline_w(fx[0], oi), bspline_w(fx[1], oj)), bspline_w(fx[2], ok));
+    const float d[3] = {__fmul_rn(__fsub_rn((float)oi, fx[0]), m.dx),
+                        __fmul_rn(__fsub_rn((float)oj, fx[1]), m.dx),
+                        __fmul_rn(__fsub_rn((float)ok, fx[2]), m.dx)};
+    float add[3];  // rounded term by term like the reference
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float ad = dot3r(affine[3 * a], affine[3 * a + 1], affine[3 * a + 2], d[0], d[1], d[2]);
+      add[a] = __fmul_rn(w, __fadd_rn(__fadd_rn(mv[a], ad), dtf[a]));
+    }
+    red_add_v4(grid + node_index(m, i, j, k), add[0], add[1], add[2], __fmul_rn(w, mass));
+    mark_block(m, dirty, i, j, k);
+  }
+}
+
+// P2G of particle p (this thread) within its CTA with the penalty coupling folded in
+// (_compute_coupling_forces_kernel, fsi/coupling.py:332-406); every thread of the CTA calls it.
+// The particle's coupling force is formed first (it is P2G's dt f term), and the fluid reaction
+// and solid fraction are spread into fa.accum beside the grid scatter, which goes to a tile of
+// nodes in shared memory. For launches of few particles only, where one launch less counts.
+// Its loop of 27 paced steps also fixes the order in which CTAs reach a node in practice: over 47
+// pairs of equal three-step runs of the 4,096-particle smoke scene the lattices were the same bit
+// for bit, against 15 pairs that differ when the coupling is a kernel of its own, and 3 to 14 of
+// 23 with P2G in runs here (which takes 12 to 15 us for this launch's 27).
+__device__ __forceinline__ void coupled_p2g_tile_body(const Mpm& m, const PView& P,
+                                                      float4* __restrict__ grid,
+                                                      uint8_t* __restrict__ dirty, int p,
+                                                      const ForceArgs& fa) {
+  __shared__ float tile[4][kTileCap];
   __shared__ int sh[8];
   const long long cap = m.cap;
   const bool act = p < m.n && P.active[p] != 0;
@@ -298,12 +602,12 @@ __device__ __forceinline__ void p2g_body(const Mpm& m, const PView& P, float4* _
   // coupling: in-grid fluid stencil nodes (bit 9i + 3j + k), valid weight, force, volume
   uint32_t usable = 0;
   float valid = 0.f, pf[3] = {0.f, 0.f, 0.f}, vp = 0.f;
-  if (kCoupled) {
+  {
     bool partial = false, clipped = false, unsupported = false;
     if (act) {
       int cb[3];
       float cw[3][3];
-      if (!coupling_particle<false>(*fa, p, cb, cw, usable, valid, pf, partial, clipped,
+      if (!coupling_particle<false>(fa, p, cb, cw, usable, valid, pf, partial, clipped,
                                     unsupported)) {
         usable = 0;
         pf[0] = pf[1] = pf[2] = 0.f;
@@ -312,9 +616,9 @@ __device__ __forceinline__ void p2g_body(const Mpm& m, const PView& P, float4* _
     } else if (p < m.n) {
       P.fp[p] = 0.f; P.fp[cap + p] = 0.f; P.fp[2 * cap + p] = 0.f;
     }
-    warp_count(&fa->cnt->unsupported, unsupported);
-    warp_count(&fa->cnt->partial, partial);
-    warp_count(&fa->cnt->clipped, clipped);
+    warp_count(&fa.cnt->unsupported, unsupported);
+    warp_count(&fa.cnt->partial, partial);
+    warp_count(&fa.cnt->clipped, clipped);
   }
   if (act) {
     float x[3];
@@ -324,7 +628,7 @@ __device__ __forceinline__ void p2g_body(const Mpm& m, const PView& P, float4* _
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       mv[a] = __fmul_rn(mass, P.v[a * cap + p]);
-      dtf[a] = __fmul_rn(m.dt, kCoupled ? pf[a] : P.fp[a * cap + p]);
+      dtf[a] = __fmul_rn(m.dt, pf[a]);
     }
   }
 
@@ -389,10 +693,10 @@ __device__ __forceinline__ void p2g_body(const Mpm& m, const PView& P, float4* _
           }
           const float addm = __fmul_rn(w, mass);
           const long long t = t0 + oa[0][si] * st0 + oa[1][sj] * st1 + oa[2][sk];
-          if (kCoupled && ((usable >> (9 * oa[0][si] + 3 * oa[1][sj] + oa[2][sk])) & 1u)) {
-            float4 c = coupling_spread_terms(fa->c, w, valid, pf, vp);
-            if (!fa->c.build_fraction) c.w = 0.f;
-            red_add_v4(fa->accum + g0 + oa[0][si] * gs0 + oa[1][sj] * m.nz + oa[2][sk],
+          if ((usable >> (9 * oa[0][si] + 3 * oa[1][sj] + oa[2][sk])) & 1u) {
+            float4 c = coupling_spread_terms(fa.c, w, valid, pf, vp);
+            if (!fa.c.build_fraction) c.w = 0.f;
+            red_add_v4(fa.accum + g0 + oa[0][si] * gs0 + oa[1][sj] * m.nz + oa[2][sk],
                        c.x, c.y, c.z, c.w);
           }
           if (use_tile) {
@@ -451,7 +755,8 @@ __device__ __forceinline__ void grid_op(const Mpm& m, float4 node, int i, int j,
 }
 
 // Grid update + G2P of particle p (this thread) within its CTA; every thread calls it.
-// kExtTile as for p2g_body (3 x kTileCap floats of the caller's shared memory).
+// kExtTile: the tile is the caller's shared memory `ext` (3 x kTileCap floats) instead of a
+// static array of its own.
 template <bool kExtTile = false>
 __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
                                          const float4* FSI_LAUNCH_RO grid, int p,

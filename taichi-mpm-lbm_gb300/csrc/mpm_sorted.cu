@@ -113,35 +113,6 @@ size_t carve(const SortGeo& g, long long cap, char* base, Work& w) {
   return off;
 }
 
-// ------------------------------------------------------------------ scans --
-// Exclusive scan over the block (blockDim.x a multiple of 32, at most 1024 threads).
-// `ws` is 32 ints of shared scratch; *total receives the block's sum.
-__device__ int block_excl_scan(int v, int* ws, int* total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) ws[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    int s = lane < nw ? ws[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += t;
-    }
-    ws[lane] = s;
-  }
-  __syncthreads();
-  const int excl = incl - v + (wid > 0 ? ws[wid - 1] : 0);
-  *total = ws[nw - 1];
-  __syncthreads();
-  return excl;
-}
-
 // 1. Base cell slot and tile count of every active particle, and the marks on the node tiles
 // of its stencil; zeroes the step counters and the list lengths.
 __global__ void __launch_bounds__(kBlock) sort_count_kernel(Mpm m, PView P, SortGeo g, Work w,
@@ -630,22 +601,6 @@ int num_sms() {
   return sms;
 }
 
-// Opts the partials kernel into its dynamic shared memory, once per device.
-template <bool kCoupled>
-int partials_smem_attr() {
-  static bool done[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return check_launch("cudaGetDevice");
-  if (dev < 0 || dev >= 64 || !done[dev]) {
-    if (cudaFuncSetAttribute(sorted_partials_kernel<kCoupled>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPartialSmem) !=
-        cudaSuccess)
-      return check_launch("cudaFuncSetAttribute(sorted_partials_kernel)");
-    if (dev >= 0 && dev < 64) done[dev] = true;
-  }
-  return FSI_OK;
-}
-
 int check_workspace(const Mpm& m, void* work, int64_t work_bytes, SortGeo& g, Work& w) {
   FSI_REQUIRE(work, "NULL workspace");
   FSI_REQUIRE(((uintptr_t)work & 255) == 0, "workspace must be 256-byte aligned");
@@ -662,7 +617,7 @@ int check_workspace(const Mpm& m, void* work, int64_t work_bytes, SortGeo& g, Wo
 template <bool kCoupled>
 int sorted_substep(const Mpm& m, const PView& P, const SortGeo& g, const Work& w, float4* grid,
                    const ForceArgs& fa, cudaStream_t s) {
-  if (int e = partials_smem_attr<kCoupled>()) return e;
+  if (int e = opt_in_smem<sorted_partials_kernel<kCoupled>>((int)kPartialSmem)) return e;
   const unsigned pg = grid_for(m.n, kBlock);
   const int sms = num_sms();
   sort_count_kernel<<<pg, kBlock, 0, s>>>(m, P, g, w, kCoupled ? fa.cnt : nullptr);

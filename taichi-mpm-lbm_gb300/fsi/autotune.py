@@ -120,7 +120,7 @@ def coupled_signature(sim) -> str:
 
 def coupled_candidates(sim) -> list[tuple[int, int]]:
     """(threads per block of P2G / G2P, coupling placement) pairs of the tiled (atomic)
-    scatter: 128, 256 or 512 particles share a shared-memory tile; the coupling force is formed
+    scatter: 128, 256 or 512 particles share a block; the coupling force is formed
     inside P2G (1), by its own kernel first (2), or by a force kernel and a spread kernel (3).
     The sorted scatter has no such choice."""
     if sim.config.mpm.p2g_mode == "sorted":

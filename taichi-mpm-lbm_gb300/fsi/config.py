@@ -156,7 +156,7 @@ class MPMConfig:
     # fixed-corotated (mpm3d.py:247-251); "neo_hookean" selects mu (F F^T - I) + lam ln(J) I.
     constitutive_model: Literal["fixed_corotated", "neo_hookean"] = "fixed_corotated"
     # Extension (no reference counterpart): how P2G sums the grid. "atomic" (default, the
-    # faster on coupled steps) scatters through shared-memory tiles with atomics, so sums
+    # faster on coupled steps) adds each thread block's node sums with atomics, so sums
     # arrive in scheduling order like the reference's parallel loop; "sorted" sorts the
     # particles by cell each substep and adds every node's contributions in one fixed order
     # (atomic-free, bit-reproducible from run to run).

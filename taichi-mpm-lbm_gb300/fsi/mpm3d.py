@@ -3,8 +3,9 @@
 Particles are stored as structure-of-arrays torch CUDA tensors (x, v, force
 ``[3, capacity]``; C, F ``[9, capacity]``; mass, volume, active ``[capacity]``)
 and advanced by the library's sm_103a substep. The default ("atomic" p2g_mode)
-scatters through shared-memory tiles with atomics and keeps the float4 grid
-all-zero between substeps by clearing only the node blocks that were touched;
+sums each thread block's particles by cell on chip, adds the sums with vector
+reductions and keeps the float4 grid all-zero between substeps by clearing only
+the node blocks that were touched;
 "sorted" sorts the particles by cell every substep and sums each grid node's
 contributions in one fixed order with plain stores (bit-reproducible). The grid
 update is fused into G2P in both.
