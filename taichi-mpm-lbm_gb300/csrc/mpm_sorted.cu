@@ -9,7 +9,8 @@
 //   2. tiles:    a two-pass scan of the tile counts (tile starts); the non-empty cell tiles and
 //                the marked node tiles are listed, and counts and marks reset for the next
 //                substep.
-//   3. cells:    per non-empty tile, a block scans its 512 cell counts (cell starts).
+//   3. cells:    per non-empty tile, a block scans its 512 cell counts (cell starts) and lists
+//                its non-empty triples of cells along z.
 //   4. scatter:  per particle, its index into its cell's range (arrival order).
 //   5. prepare:  per particle, its rank in the cell (ascending particle index) gives its
 //                sorted position; the coupling force (interpolated fluid velocity, penalty,
@@ -18,9 +19,9 @@
 //                are written to the payload at the sorted position.
 //   6. partials: per non-empty cell b and stencil offset o, the sum of the cell's particles'
 //                contributions to node b + o in ascending particle index (and, coupled, the
-//                reaction / solid-fraction sum of its coupled particles): one block per
-//                non-empty cell tile, a warp per z-run of three cells, particles staged in
-//                shared memory by asynchronous copies one chunk ahead of the arithmetic.
+//                reaction / solid-fraction sum of its coupled particles): a warp per triple of
+//                cells from a list of the non-empty ones, particles staged in shared memory
+//                by asynchronous copies one chunk ahead of the arithmetic.
 //   7. nodes:    each node of a touched 8^3 node tile adds its cells' partials in ascending
 //                cell index: momentum/mass into the grid from zero, the coupling partials onto
 //                the lattice accumulator. Plain stores, no atomics, and no grid clear: the
@@ -62,7 +63,8 @@ struct Work {
   int32_t* cell_tiles;    // [ntiles] non-empty cell tiles
   int32_t* node_tiles;    // [nntiles] node tiles touched by some stencil
   uint8_t* node_flag;     // [nntiles] touched this substep, zero between substeps
-  int32_t* header;        // [0] cell tiles, [1] node tiles, [4] partials work cursor
+  int32_t* header;        // [0] cell tiles, [1] node tiles, [2] triples
+  int4* triples;          // [cap] non-empty triples of cells: their starts, the last one's end
   int32_t* key;           // [cap] tile * 512 + local cell, or -1
   int32_t* slot;          // [cap]
   int32_t* unsorted;      // [cap]
@@ -104,6 +106,7 @@ size_t carve(const SortGeo& g, long long cap, char* base, Work& w) {
   w.node_tiles = reinterpret_cast<int32_t*>(take((size_t)g.nntiles * 4));
   w.node_flag = reinterpret_cast<uint8_t*>(take((size_t)g.nntiles));
   w.header = reinterpret_cast<int32_t*>(take(64));
+  w.triples = reinterpret_cast<int4*>(take((size_t)cap * sizeof(int4)));
   w.key = reinterpret_cast<int32_t*>(take((size_t)cap * 4));
   w.slot = reinterpret_cast<int32_t*>(take((size_t)cap * 4));
   w.unsorted = reinterpret_cast<int32_t*>(take((size_t)cap * 4));
@@ -119,8 +122,7 @@ __global__ void __launch_bounds__(kBlock) sort_count_kernel(Mpm m, PView P, Sort
                                                             Cnt* cnt) {
   const int p = blockIdx.x * kBlock + threadIdx.x;
   if (p == 0) {
-    w.header[0] = 0;
-    w.header[1] = 0;
+    w.header[0] = w.header[1] = w.header[2] = 0;
     if (cnt) { cnt->unsupported = 0; cnt->partial = 0; cnt->clipped = 0; }
   }
   int key = -1, tile = -1, slot = 0;
@@ -189,21 +191,23 @@ __global__ void __launch_bounds__(kScanThreads) sort_tile_scan_global_kernel(Sor
   w.tile_count[i] = 0;
 }
 
-// 2c. The node tiles some stencil touched are listed (arrival order) and their marks reset;
-// the partials kernel's work cursor is reset.
+// 2c. The node tiles some stencil touched are listed (arrival order) and their marks reset.
 __global__ void __launch_bounds__(kBlock) sort_node_tiles_kernel(SortGeo g, Work w) {
   const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i == 0) w.header[4] = 0;
   if (i >= g.nntiles || w.node_flag[i] == 0) return;
   w.node_flag[i] = 0;
   w.node_tiles[atomicAdd(&w.header[1], 1)] = i;
 }
 
 // 3. Cell starts (and the first sorted position of each non-empty cell) of each non-empty
-// cell tile, one block of 512 threads per tile; the cell counts are reset.
+// cell tile, one block of 512 threads per tile; the cell counts are reset. The non-empty
+// triples of cells (cells 0-2, 3-5 and 6-7 of a row of eight along z) are listed for the
+// partials, in arrival order (the list only schedules work; it has at most one entry per
+// particle).
 __global__ void __launch_bounds__(kTC) sort_cell_scan_kernel(Work w) {
   __shared__ int ws[32];
   const int n = w.header[0];
+  const int lane = threadIdx.x & 31;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const int t = w.cell_tiles[i];
     const long long idx = (long long)t * kTC + threadIdx.x;
@@ -214,6 +218,22 @@ __global__ void __launch_bounds__(kTC) sort_cell_scan_kernel(Work w) {
     w.cell_start[idx] = start;
     w.cell_row[idx] = c > 0 ? start : -1;
     w.cell_count[idx] = 0;
+    // a warp holds four rows; the first lane of a triple speaks for it
+    const int z = lane & (kT - 1), cells = z == 6 ? 2 : 3;
+    const int end = start + c;
+    int4 e;
+    e.x = start;
+    e.y = __shfl_down_sync(0xffffffffu, start, 1);
+    e.z = __shfl_down_sync(0xffffffffu, start, 2);
+    const int end1 = __shfl_down_sync(0xffffffffu, end, 1), end2 = __shfl_down_sync(0xffffffffu, end, 2);
+    e.w = cells == 3 ? end2 : end1;
+    if (cells == 2) e.z = e.w;
+    const bool some = z % 3 == 0 && e.w > e.x;
+    const unsigned mask = __ballot_sync(0xffffffffu, some);
+    int at = 0;
+    if (lane == 0 && mask) at = atomicAdd(&w.header[2], __popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(mask & ((1u << lane) - 1u));
+    if (some) w.triples[at] = e;
   }
 }
 
@@ -312,37 +332,29 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Particles per cell and chunk staged in shared memory by the partials kernel, and the
-// float4 slots per staged particle (the payload's 8 plus one, which with the extra slot per
-// cell area puts the three cells of a warp on different shared-memory banks).
-constexpr int kChunk = 8;
-constexpr int kSlot = kPay + 1;
+// Particles per cell and chunk staged in shared memory by the partials kernel: 8 per cell is
+// the usual density, 11 keeps a cell that a deforming body crowds in one chunk, and three
+// blocks on an SM. Lanes of a cell read one particle at a time; the extra float4 per cell area
+// puts the three cells of a warp on different shared-memory banks.
+constexpr int kChunk = 11;
+constexpr int kSlot = kPay;
 constexpr int kGroupF4 = kChunk * kSlot + 1;  // one cell's staging area, in float4
 constexpr int kWarpBufF4 = 3 * kGroupF4;      // three cells
 constexpr int kPartialWarps = kTileThreads / 32;
-constexpr size_t kPartialSmem =
-    (size_t)2 * kPartialWarps * kWarpBufF4 * sizeof(float4) + kTC * sizeof(int2);
+constexpr size_t kPartialSmem = (size_t)2 * kPartialWarps * kWarpBufF4 * sizeof(float4);
 
-// One triple of cells of a cell tile: a z-run (cells lz = 3 r, 3 r + 1, 3 r + 2 of row
-// (lx, ly)); the lanes 9 g .. 9 g + 8 of a warp serve cell g of the triple.
+// A listed triple of cells: the lanes 9 g .. 9 g + 8 of a warp serve cell g.
 struct Triple {
-  int start, count;  // this lane's cell (count 0: no cell or empty)
+  int start, count;  // this lane's cell
   int maxcount;      // warp-wide
 };
 
-// cells: the tile's (start, count) per local cell, staged in shared memory.
-__device__ __forceinline__ Triple load_triple(const int2* cells, int tr, int grp) {
-  Triple t;
-  t.start = 0;
-  t.count = 0;
-  const int row = tr / 3, lz = 3 * (tr % 3) + grp;
-  if (grp < 3 && lz < kT) {
-    const int2 c = cells[row * kT + lz];
-    t.start = c.x;
-    t.count = c.y;
-  }
-  t.maxcount = __reduce_max_sync(0xffffffffu, t.count);
-  return t;
+__device__ __forceinline__ Triple triple_of(const int4& e, int grp) {
+  Triple r;
+  r.start = grp == 0 ? e.x : (grp == 1 ? e.y : e.z);
+  r.count = grp < 3 ? (grp == 0 ? e.y : (grp == 1 ? e.z : e.w)) - r.start : 0;
+  r.maxcount = max(e.y - e.x, max(e.z - e.y, e.w - e.z));
+  return r;
 }
 
 // Stages particles [chunk * kChunk, ...) of the warp's three cells into buf (all lanes copy).
@@ -374,46 +386,30 @@ __device__ __forceinline__ void stage_chunk(const Work& w, float4* buf, int lane
 // 6. Cell partials: for every non-empty cell b and stencil offset o, the sum over the cell's
 // particles (ascending index, from zero) of their contribution to node b + o, written to
 // partial[cell_row(b) * 27 + o]; the coupling partial (reaction, solid fraction) sums the
-// cell's coupled particles. A block takes non-empty cell tiles from a cursor; a warp handles
-// z-runs of three cells, their particles staged in shared memory with asynchronous copies one
-// chunk ahead of the arithmetic. Lane (g, ox, oy) forms the partials of offsets (ox, oy, 0..2)
-// of cell g, which share the x and y factors of the weight and the first two terms of the
-// affine product.
+// cell's coupled particles. A warp takes triples of cells from the list, grid-stride, their
+// particles staged in shared memory with asynchronous copies one chunk ahead of the arithmetic,
+// across triples. Lane (g, ox, oy) forms the partials of offsets (ox, oy, 0..2) of cell g, which
+// share the x and y factors of the weight and the first two terms of the affine product.
+// Why a list of triples: a body of 11^3 cells lies in 27 tiles, so with a block per tile most of
+// the chip idled while 8 warps walked up to 4,096 particles one after another: 114 us for the
+// 52,000 particles of seven bodies. With a warp per row of eight cells, three quarters of them
+// empty, 38 us; with listed triples 21 us. Nothing here is shared by a block: no barriers.
 template <bool kCoupled>
 __global__ void __launch_bounds__(kTileThreads, kCoupled ? 2 : 3)
     sorted_partials_kernel(Mpm m, Work w, fsi_coupling_desc cd) {
   constexpr int NC = kCoupled ? 2 : 1;
   extern __shared__ float4 smem[];
-  __shared__ int next_tile;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float4* bufs = smem + (size_t)warp * 2 * kWarpBufF4;
-  int2* cells = reinterpret_cast<int2*>(smem + (size_t)2 * kPartialWarps * kWarpBufF4);
   const int grp = lane / 9, r9 = lane - 9 * grp;
   const int ox = r9 / 3, oy = r9 - 3 * ox;
   const int gsel = grp < 3 ? grp : 0;
-  const int ntiles = w.header[0];
-  constexpr int kTriples = kT * kT * 3;  // (lx, ly) rows x three z-runs
-  for (;;) {
-    __syncthreads();  // the previous tile's cell table and cursor are no longer read
-    if (threadIdx.x == 0) next_tile = atomicAdd(&w.header[4], 1);
-    __syncthreads();
-    const int ti = next_tile;
-    if (ti >= ntiles) break;
-    const int tile = w.cell_tiles[ti];
-    for (int c = threadIdx.x; c < kTC; c += kTileThreads) {
-      const int key = tile * kTC + c;
-      const int st = w.cell_start[key];
-      cells[c] = make_int2(st, cell_end(w, key) - st);
-    }
-    __syncthreads();
-    // Job sequence of this warp: (triple, chunk) pairs of its non-empty triples, in order.
-    int tr = warp;
-    Triple cur;
-    for (; tr < kTriples; tr += kPartialWarps) {
-      cur = load_triple(cells, tr, grp);
-      if (cur.maxcount > 0) break;
-    }
-    if (tr >= kTriples) continue;
+  const int n = w.header[2];
+  const int stride = gridDim.x * kPartialWarps;
+  // neighbouring triples go to different blocks, so few of them still fill the chip
+  int j = warp * gridDim.x + blockIdx.x;
+  if (j < n) {
+    Triple cur = triple_of(w.triples[j], grp);
     int chunk = 0, slot = 0;
     stage_chunk(w, bufs, lane, cur.start, cur.count, 0);
     float am[3][4], ac[3][4];
@@ -424,16 +420,14 @@ __global__ void __launch_bounds__(kTileThreads, kCoupled ? 2 : 3)
     bool any_coupled = false;
     for (;;) {
       // The next job, whose copies go out before this job's arithmetic.
-      int ntr = tr, nchunk = chunk + 1;
+      int nj = j, nchunk = chunk + 1;
       Triple nxt = cur;
       if (nchunk * kChunk >= cur.maxcount) {
         nchunk = 0;
-        for (ntr = tr + kPartialWarps; ntr < kTriples; ntr += kPartialWarps) {
-          nxt = load_triple(cells, ntr, grp);
-          if (nxt.maxcount > 0) break;
-        }
+        nj = j + stride;
+        if (nj < n) nxt = triple_of(w.triples[nj], grp);
       }
-      const bool more = ntr < kTriples;
+      const bool more = nj < n;
       if (more) stage_chunk(w, bufs + (slot ^ 1) * kWarpBufF4, lane, nxt.start, nxt.count, nchunk);
       if (more) cp_async_wait<1>(); else cp_async_wait<0>();
       __syncwarp();
@@ -497,7 +491,7 @@ __global__ void __launch_bounds__(kTileThreads, kCoupled ? 2 : 3)
         any_coupled = false;
       }
       if (!more) break;
-      tr = ntr;
+      j = nj;
       chunk = nchunk;
       cur = nxt;
       slot ^= 1;
@@ -555,11 +549,19 @@ __global__ void __launch_bounds__(kTC, 2) sorted_nodes_kernel(Mpm m, SortGeo g, 
       const int i = ij / 3, j = ij % 3;
       const int* rr = region + ((x + 2 - i) * kRE + (y + 2 - j)) * kRE + z;
       const int rows[3] = {rr[0], rr[1], rr[2]};  // k = 2, 1, 0
-      float4 pm[3];
+      float4 pm[3], sc[3];
+      bool cpl[3];
 #pragma unroll
-      for (int t3 = 0; t3 < 3; ++t3)
-        pm[t3] = rows[t3] >= 0 ? w.partial[((long long)rows[t3] * 27 + 3 * ij + 2 - t3) * NC]
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int t3 = 0; t3 < 3; ++t3) {
+        const float4* src = w.partial + ((long long)rows[t3] * 27 + 3 * ij + 2 - t3) * NC;
+        pm[t3] = rows[t3] >= 0 ? src[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+        cpl[t3] = false;
+        // loaded beside the flag that says whether it counts, not after it
+        if (kCoupled && rows[t3] >= 0) {
+          sc[t3] = src[1];
+          cpl[t3] = fluid && w.cell_coupled[rows[t3]] != 0;
+        }
+      }
 #pragma unroll
       for (int t3 = 0; t3 < 3; ++t3) {
         if (rows[t3] < 0) continue;
@@ -567,12 +569,11 @@ __global__ void __launch_bounds__(kTC, 2) sorted_nodes_kernel(Mpm m, SortGeo g, 
         am.y = __fadd_rn(am.y, pm[t3].y);
         am.z = __fadd_rn(am.z, pm[t3].z);
         am.w = __fadd_rn(am.w, pm[t3].w);
-        if (kCoupled && fluid && w.cell_coupled[rows[t3]]) {
-          const float4 sc = w.partial[((long long)rows[t3] * 27 + 3 * ij + 2 - t3) * NC + 1];
-          ac.x = __fadd_rn(ac.x, sc.x);
-          ac.y = __fadd_rn(ac.y, sc.y);
-          ac.z = __fadd_rn(ac.z, sc.z);
-          if (cd.build_fraction) ac.w = __fadd_rn(ac.w, sc.w);
+        if (kCoupled && cpl[t3]) {
+          ac.x = __fadd_rn(ac.x, sc[t3].x);
+          ac.y = __fadd_rn(ac.y, sc[t3].y);
+          ac.z = __fadd_rn(ac.z, sc[t3].z);
+          if (cd.build_fraction) ac.w = __fadd_rn(ac.w, sc[t3].w);
         }
       }
     }
@@ -640,7 +641,8 @@ int sorted_substep(const Mpm& m, const PView& P, const SortGeo& g, const Work& w
   else
     sorted_prepare_kernel<kCoupled, false><<<pg, kBlock, 0, s>>>(m, P, w, fa);
   if (int e = check_launch("sorted_prepare_kernel")) return e;
-  const int pb = g.ntiles < 3 * sms ? g.ntiles : 3 * sms;
+  const int pb = (int)grid_for((m.n + 7) / 8, kPartialWarps) < 3 * sms
+                     ? (int)grid_for((m.n + 7) / 8, kPartialWarps) : 3 * sms;
   sorted_partials_kernel<kCoupled><<<pb, kTileThreads, kPartialSmem, s>>>(m, w, fa.c);
   if (int e = check_launch("sorted_partials_kernel")) return e;
   const int nb = g.nntiles < 4 * sms ? g.nntiles : 4 * sms;

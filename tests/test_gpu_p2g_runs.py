@@ -69,3 +69,24 @@ def test_runs_against_oracle(case, threads):
         o.substep()
     assert rel_l2(g.velocities_numpy(), o.velocities_numpy()) < 1e-3
     assert rel_l2(g.positions_numpy(), o.positions_numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("per_cell", [1, 10, 11, 12, 22, 23])
+def test_sorted_chunks_and_triples_bit_exact(per_cell):
+    """The sorted scatter's listed triples of cells at every place of a row of eight along z, with
+    counts around the chunk that is staged at a time (11), bit for bit the oracle's cell order."""
+    rng = np.random.default_rng(per_cell)
+    cells = [(4, 5, z) for z in range(3, 22)] + [(6, 8, z) for z in (3, 5, 6, 9, 12, 14, 15)] + [(9, 9, 13)]
+    pos = np.concatenate([np.asarray(c) + rng.uniform(0.55, 1.45, (per_cell, 3)) for c in cells])
+    pos = pos[rng.permutation(len(pos))].astype(np.float32)
+    vel = rng.normal(0, 1e-2, pos.shape).astype(np.float32)
+    cfg = MPMConfig(nx=17, ny=18, nz=27, max_particles=1000, dt=1e-2, youngs_modulus=100.0,
+                    gravity=(0.0, -1e-3, 0.0), boundary_width=2, p2g_mode="sorted")
+    g, o = MPMSolver3D(cfg), O.MPMSolver3D(cfg, polar="device", cell_order=True)
+    for s in (g, o):
+        s.initialize_particles_from_numpy(pos, vel, particle_volume=0.125)
+    for _ in range(3):
+        g.substep()
+        o.substep()
+        np.testing.assert_array_equal(g.velocities_numpy(), o.velocities_numpy())
+        np.testing.assert_array_equal(g.positions_numpy(), o.positions_numpy())
