@@ -681,6 +681,42 @@ int fsi_closure_colsum(const void* g, int32_t m, int32_t n, float* out, void* st
 int fsi_closure_adam(float* params, const float* grads, float* m, float* v, int64_t n, float lr,
                      float beta1, float beta2, float eps, int32_t step, void* stream);
 
+/* One training step of the network on a mini-batch, in one call: rows index[i] of x (BF16
+ * [..][656]) and target (FP32 [..][19]) are picked, then forward pass, mean-square loss, all
+ * gradients (into grads, overwritten), one bias-corrected Adam step of params, and the BF16
+ * copies of the new weights (w2t, w3t, w4t their transposes [64][64], [64][64], [64][32]; bias =
+ * b1 b2 b3 b4). params, grads, adam_m, adam_v: FP32, W1 [64][656], b1 [64], W2 [64][64], b2, W3
+ * [64][64], b3, W4 [32][64], b4 [32]. m: rows, a multiple of 128. index values must be rows of x
+ * and target. loss: device double, set to the batch's loss. work: scratch of
+ * fsi_closure_train_bytes(m) bytes, 256-byte aligned. Nothing is kept after the call. */
+typedef struct fsi_closure_train_desc {
+  const void* x;
+  const float* target;
+  const int64_t* index;
+  float* params;
+  float* grads;
+  float* adam_m;
+  float* adam_v;
+  void* w1;
+  void* w2;
+  void* w3;
+  void* w4;
+  void* w2t;
+  void* w3t;
+  void* w4t;
+  float* bias;
+  void* work;
+  int64_t work_bytes;
+  double* loss;
+  int32_t* err;
+  int32_t m;
+  int32_t step; /* Adam's step count, from 1 */
+  float lr, beta1, beta2, eps;
+} fsi_closure_train_desc;
+/* Scratch bytes of a training step of m rows, or -1 when m is not a positive multiple of 128. */
+int64_t fsi_closure_train_bytes(int32_t m);
+int fsi_closure_train_step(const fsi_closure_train_desc* desc, void* stream);
+
 /* Self-test of the bounded mbarrier waits of the tensor-core kernels (no reference
  * counterpart; a failure-detection check that faults nothing). One CTA waits on a barrier that
  * nothing arrives on: out[0] = 0 when the plain wait gave up after its clock limit (about one

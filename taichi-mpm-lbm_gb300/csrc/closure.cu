@@ -15,7 +15,7 @@
 // Kernels:
 //   closure_features_kernel: the feature rows of a list of cells, BF16 [M][656] (training).
 //   gemm_kernel: C = A B^T for K-major BF16 A [M][K], B [N][K] (row-major in global memory),
-//     128-row tiles, split-K over blockIdx.y, two-stage cp.async pipeline into shared memory
+//     128-row tiles, split-K over blockIdx.y, three- or four-stage cp.async pipeline into shared memory
 //     (canonical no-swizzle core-matrix layout), tcgen05.mma into tensor memory, and a fused
 //     epilogue: store FP32 / add FP32 atomically / bias + GELU forward (BF16 activations,
 //     their transpose and the FP32 pre-activation) / GELU backward (BF16 gradient and its
@@ -149,12 +149,39 @@ struct GemmArgs {
 
 constexpr int kBM = 128, kBK = 64;
 
+// Chunks of K in flight: a block's whole loop is a handful of chunks (11 for K = 656), each a
+// round trip to L2 or HBM, so the loop is bound by how many of them overlap. 128 columns take
+// 32 KB a chunk, and three of them leave room for two blocks on an SM.
+template <int BN>
+constexpr int gemm_stages() { return BN == 128 ? 3 : 4; }
+template <int BN>
+constexpr int gemm_smem() { return gemm_stages<BN>() * (kBM + BN) * kBK * 2; }
+
+// 16 consecutive columns c0.. of row r of the epilogue, as vectors: every thread holds a row, so
+// scalar accesses would touch 32 sectors per warp for 2 or 4 bytes each.
+__device__ __forceinline__ void store_bf16x16(__nv_bfloat16* p, const float (&v)[16]) {
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const __nv_bfloat162 pr = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    w[i] = *reinterpret_cast<const uint32_t*>(&pr);
+  }
+  reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+__device__ __forceinline__ void store_f32x16(float* p, const float (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    reinterpret_cast<float4*>(p)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+
 template <int BN>
 __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
+  constexpr int kST = gemm_stages<BN>();
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* sa[2] = {smem, smem + kBM * kBK * 2};
-  unsigned char* sb[2] = {smem + 2 * kBM * kBK * 2, smem + 2 * kBM * kBK * 2 + BN * kBK * 2};
-  __shared__ __align__(8) uint64_t bar[2];
+  auto sa = [&](int s) { return smem + s * (kBM + BN) * kBK * 2; };
+  auto sb = [&](int s) { return smem + s * (kBM + BN) * kBK * 2 + kBM * kBK * 2; };
+  __shared__ __align__(8) uint64_t bar[kST];
   __shared__ uint32_t tbase;
   const int t = threadIdx.x, warp = t >> 5;
   const int row0 = blockIdx.x * kBM, col0 = blockIdx.z * BN;
@@ -163,79 +190,120 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
   const int nk = (kend - kbeg + kBK - 1) / kBK;
 
   if (warp == 0) tc::tmem_alloc(&tbase, BN < 32 ? 32 : BN);
-  if (t == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); }
+  if (t == 0) {
+    for (int s = 0; s < kST; ++s) tc::mbar_init(&bar[s], 1);
+  }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tbase;
 
-  // Copies K chunk `c` of A and B into stage s (16-byte pieces; zero-fill outside).
-  auto load = [&](int c, int s) {
-    const int k0 = kbeg + c * kBK;
-    const uint32_t a0 = tc::smem_addr(sa[s]), b0 = tc::smem_addr(sb[s]);
-    for (int p = t; p < kBM * (kBK / 8); p += 128) {
-      const int r = p / (kBK / 8), kk = (p % (kBK / 8)) * 8;
-      const bool ok = row0 + r < g.m && k0 + kk < kend;
-      const __nv_bfloat16* src = g.A + (size_t)(ok ? row0 + r : 0) * g.lda + (ok ? k0 + kk : 0);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a0 + tc::kmajor_offset(r, kk, kBK)),
-                   "l"(src), "r"(ok ? 16 : 0));
-    }
-    for (int p = t; p < BN * (kBK / 8); p += 128) {
-      const int r = p / (kBK / 8), kk = (p % (kBK / 8)) * 8;
-      const bool ok = col0 + r < g.n && k0 + kk < kend;
-      const __nv_bfloat16* src = g.B + (size_t)(ok ? col0 + r : 0) * g.ldb + (ok ? k0 + kk : 0);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(b0 + tc::kmajor_offset(r, kk, kBK)),
-                   "l"(src), "r"(ok ? 16 : 0));
+  // Copies K chunk `c` of A and B into its stage (16-byte pieces; zero-fill outside) and closes
+  // the copy group of chunk c, an empty one past the end.
+  auto load = [&](int c) {
+    if (c < nk) {
+      const int k0 = kbeg + c * kBK;
+      const uint32_t a0 = tc::smem_addr(sa(c % kST)), b0 = tc::smem_addr(sb(c % kST));
+      for (int p = t; p < kBM * (kBK / 8); p += 128) {
+        const int r = p / (kBK / 8), kk = (p % (kBK / 8)) * 8;
+        const bool ok = row0 + r < g.m && k0 + kk < kend;
+        const __nv_bfloat16* src = g.A + (size_t)(ok ? row0 + r : 0) * g.lda + (ok ? k0 + kk : 0);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a0 + tc::kmajor_offset(r, kk, kBK)),
+                     "l"(src), "r"(ok ? 16 : 0));
+      }
+      for (int p = t; p < BN * (kBK / 8); p += 128) {
+        const int r = p / (kBK / 8), kk = (p % (kBK / 8)) * 8;
+        const bool ok = col0 + r < g.n && k0 + kk < kend;
+        const __nv_bfloat16* src = g.B + (size_t)(ok ? col0 + r : 0) * g.ldb + (ok ? k0 + kk : 0);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(b0 + tc::kmajor_offset(r, kk, kBK)),
+                     "l"(src), "r"(ok ? 16 : 0));
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
   bool ok = true;
-  uint32_t uses[2] = {0, 0};
-  if (nk > 0) load(0, 0);
-  for (int c = 0; c < nk && ok; ++c) {
-    const int s = c & 1;
-    if (c + 1 < nk) {
-      const int s2 = (c + 1) & 1;
-      if (c + 1 >= 2) {  // the MMAs that read stage s2 (chunk c - 1) must be done
-        // One decision for the whole CTA: the loop body holds block-wide barriers.
-        ok = __syncthreads_and(tc::mbar_wait(&bar[s2], (uses[s2] - 1) & 1, g.err, 1)) != 0;
-        if (!ok) break;
-      }
-      load(c + 1, s2);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+  for (int c = 0; c < kST - 1; ++c) load(c);
+  for (int c = 0; c < nk; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kST - 2) : "memory");  // chunk c has arrived
     tc::fence_smem_for_async();
     tc::fence_before_sync();
     __syncthreads();
     if (t == 0) {
       tc::fence_after_sync();
-      const uint32_t a0 = tc::smem_addr(sa[s]), b0 = tc::smem_addr(sb[s]);
+      const uint32_t a0 = tc::smem_addr(sa(c % kST)), b0 = tc::smem_addr(sb(c % kST));
 #pragma unroll
       for (int q = 0; q < kBK / 16; ++q)
         tc::mma_bf16(tmem, tc::tile_desc(a0, kBK, q), tc::tile_desc(b0, kBK, q),
                      tc::idesc_bf16(kBM, BN), c > 0 || q > 0);
-      tc::mma_commit(&bar[s]);
+      tc::mma_commit(&bar[c % kST]);
     }
-    ++uses[s];
+    // Chunk c + kST - 1 goes where chunk c - 1 was, once the MMAs that read it are done. One
+    // decision for the whole CTA: the loop body holds block-wide barriers.
+    if (c > 0 && c + kST - 1 < nk) {
+      ok = __syncthreads_and(tc::mbar_wait(&bar[(c - 1) % kST], ((c - 1) / kST) & 1, g.err, 1)) != 0;
+      if (!ok) break;
+    }
+    load(c + kST - 1);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   // All MMAs were committed in order: the last commit completes after all of them.
-  if (ok && nk > 0) {
-    const int s = (nk - 1) & 1;
-    ok = tc::mbar_wait(&bar[s], (uses[s] - 1) & 1, g.err, 2);
-  }
+  if (ok && nk > 0) ok = tc::mbar_wait(&bar[(nk - 1) % kST], ((nk - 1) / kST) & 1, g.err, 2);
   ok = __syncthreads_and(ok) != 0;  // the epilogue's TMEM loads are warp-collective
   tc::fence_after_sync();
   const int r = row0 + 32 * warp + (t & 31);
+  // whole groups of 16 columns at 16-byte boundaries go as vectors
+  const bool vec_c = (g.ldc & 3) == 0 && ((uintptr_t)g.C & 15) == 0;
+  const bool vec_h = (g.n & 7) == 0 &&
+                     (((uintptr_t)g.H | (uintptr_t)g.Zout | (uintptr_t)g.Zin) & 15) == 0;
   if (ok && nk > 0) {
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 16) {
       float v[16];
       tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c0, v);  // whole warp
       if (r >= g.m) continue;
+      const int first = col0 + c0;
+      const bool whole = first + 16 <= g.n;
+      if (whole && g.mode <= kAtomicF32 && vec_c) {
+        float* c = g.C + (size_t)r * g.ldc + first;
+        if (g.mode == kStoreF32) {
+          store_f32x16(c, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; i += 4)
+            red_add_v4(reinterpret_cast<float4*>(c + i), v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        continue;
+      }
+      if (whole && g.mode >= kGeluFwd && vec_h) {
+        const size_t at = (size_t)r * g.n + first;
+        float h[16];
+        if (g.mode == kGeluFwd) {
+          float z[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            z[i] = v[i] + g.bias[first + i];
+            h[i] = gelu(z[i]);
+          }
+          if (g.Zout) store_f32x16(g.Zout + at, z);
+        } else {
+          const float4* zi = reinterpret_cast<const float4*>(g.Zin + at);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 z = zi[i];
+            h[4 * i] = v[4 * i] * gelu_grad(z.x);
+            h[4 * i + 1] = v[4 * i + 1] * gelu_grad(z.y);
+            h[4 * i + 2] = v[4 * i + 2] * gelu_grad(z.z);
+            h[4 * i + 3] = v[4 * i + 3] * gelu_grad(z.w);
+          }
+        }
+        store_bf16x16(g.H + at, h);
+        if (g.HT) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) g.HT[(size_t)(first + i) * g.ldht + r] = __float2bfloat16_rn(h[i]);
+        }
+        continue;
+      }
       for (int i = 0; i < 16; ++i) {
         const int col = col0 + c0 + i;
         if (col >= g.n) break;
@@ -957,35 +1025,83 @@ __global__ void __launch_bounds__(kBlock) closure_restrict_kernel(LbmGeom fg, co
 }
 
 // dY = 2 (Y + b4 - T) / (m * 19) on the 19 outputs (0 on padding), BF16 [m][32] and its
-// transpose [32][ldt]; loss += sum (Y + b4 - T)^2 / (m * 19).
+// transpose [32][ldt]; loss += sum (Y + b4 - T)^2 / (m * 19). A block takes 64 rows; the
+// transpose goes through shared memory, and each block adds its part of the loss once (one
+// addition per warp on one address, and 2-byte stores a row apart, took 28 us for 16,384 rows).
+constexpr int kLossRows = 64;
 __global__ void __launch_bounds__(kBlock) closure_loss_kernel(const float* __restrict__ y,
                                                               const float* __restrict__ target,
                                                               const float* __restrict__ b4, int m,
                                                               __nv_bfloat16* __restrict__ dy,
                                                               __nv_bfloat16* __restrict__ dyt, int ldt,
                                                               double* __restrict__ loss) {
-  const long long t = (long long)blockIdx.x * kBlock + threadIdx.x;
+  __shared__ __nv_bfloat16 tr[kLossRows][kOutPad + 2];
+  __shared__ double part[kBlock / 32];
+  const int r0 = blockIdx.x * kLossRows;
   float e2 = 0.f;
-  if (t < (long long)m * kOutPad) {
-    const int r = (int)(t / kOutPad), q = (int)(t % kOutPad);
+  for (int i = threadIdx.x; i < kLossRows * kOutPad; i += kBlock) {
+    const int rl = i / kOutPad, q = i % kOutPad, r = r0 + rl;
     float gq = 0.f;
-    if (q < kOut) {
-      const float e = y[t] + b4[q] - target[(size_t)r * kOut + q];
-      e2 = e * e;
+    if (r < m && q < kOut) {
+      const float e = y[(size_t)r * kOutPad + q] + b4[q] - target[(size_t)r * kOut + q];
+      e2 += e * e;
       gq = 2.f * e / ((float)m * kOut);
     }
     const __nv_bfloat16 h = __float2bfloat16_rn(gq);
-    dy[t] = h;
-    dyt[(size_t)q * ldt + r] = h;
+    tr[rl][q] = h;
+    if (r < m) dy[(size_t)r * kOutPad + q] = h;
   }
+  double d = (double)e2;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) e2 += __shfl_down_sync(0xffffffffu, e2, o);
-  if ((threadIdx.x & 31) == 0 && e2 != 0.f) atomicAdd(loss, (double)e2 / ((double)m * kOut));
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = d;
+  __syncthreads();
+  for (int i = threadIdx.x; i < kLossRows * kOutPad; i += kBlock) {
+    const int q = i / kLossRows, rl = i % kLossRows;
+    if (r0 + rl < m) dyt[(size_t)q * ldt + r0 + rl] = tr[rl][q];
+  }
+  if (threadIdx.x == 0) {
+    double sum = 0.0;
+    for (int i = 0; i < kBlock / 32; ++i) sum += part[i];
+    if (sum != 0.0) atomicAdd(loss, sum / ((double)m * kOut));
+  }
 }
 
-// out[c] += sum over rows of g[r][c] (bias gradients), g BF16 [m][n].
-__global__ void __launch_bounds__(kBlock) closure_colsum_kernel(const __nv_bfloat16* __restrict__ g,
-                                                                int m, int n, float* __restrict__ out) {
+// out[c] += sum over rows of g[r][c] (bias gradients) of up to four BF16 matrices [m][n], one per
+// blockIdx.y. Pairs of columns per thread, neighbouring threads on neighbouring pairs of a row.
+struct ColsumArgs {
+  const __nv_bfloat16* g[4];
+  float* out[4];
+  int n[4];  // even, at most 512
+};
+__global__ void __launch_bounds__(kBlock) closure_colsum_kernel(ColsumArgs a, int m) {
+  __shared__ float2 part[kBlock];
+  const int which = blockIdx.y, np = a.n[which] / 2;
+  const int rows = kBlock / np;  // rows a block reads at once
+  const int c = threadIdx.x % np, rl = threadIdx.x / np;
+  float2 s = make_float2(0.f, 0.f);
+  if (rl < rows) {
+    const __nv_bfloat162* g = reinterpret_cast<const __nv_bfloat162*>(a.g[which]);
+    for (long long r = (long long)blockIdx.x * rows + rl; r < m; r += (long long)gridDim.x * rows) {
+      const float2 v = __bfloat1622float2(g[r * np + c]);
+      s.x += v.x;
+      s.y += v.y;
+    }
+  }
+  part[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < np) {
+    for (int i = 1; i < rows; ++i) {
+      s.x += part[i * np + threadIdx.x].x;
+      s.y += part[i * np + threadIdx.x].y;
+    }
+    atomicAdd(a.out[which] + 2 * threadIdx.x, s.x);
+    atomicAdd(a.out[which] + 2 * threadIdx.x + 1, s.y);
+  }
+}
+// The same for any width: one column per block in y.
+__global__ void __launch_bounds__(kBlock) closure_colsum_any_kernel(const __nv_bfloat16* __restrict__ g,
+                                                                    int m, int n, float* __restrict__ out) {
   const int col = blockIdx.y;
   float s = 0.f;
   for (long long r = (long long)blockIdx.x * kBlock + threadIdx.x; r < m; r += (long long)gridDim.x * kBlock)
@@ -1052,6 +1168,17 @@ extern "C" int fsi_closure_features(const fsi_lbm_desc* d, const float* pops, co
   return check_launch("closure_features_kernel");
 }
 
+namespace fsi {
+namespace {
+template <int BN>
+int launch_gemm(const GemmArgs& g, dim3 grid, cudaStream_t s) {
+  if (int e = opt_in_smem<gemm_kernel<BN>>(gemm_smem<BN>())) return e;
+  gemm_kernel<BN><<<grid, 128, gemm_smem<BN>(), s>>>(g);
+  return check_launch("gemm_kernel");
+}
+}  // namespace
+}  // namespace fsi
+
 extern "C" int fsi_closure_gemm(const fsi_closure_gemm_desc* d, void* stream) {
   FSI_REQUIRE(d && d->a && d->b && d->err, "NULL GEMM operand");
   FSI_REQUIRE(d->m > 0 && d->n > 0 && d->k > 0, "empty GEMM");
@@ -1076,18 +1203,9 @@ extern "C" int fsi_closure_gemm(const fsi_closure_gemm_desc* d, void* stream) {
   const dim3 grid((d->m + kBM - 1) / kBM, (d->k + d->k_chunk - 1) / d->k_chunk, (d->n + bn - 1) / bn);
   FSI_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "GEMM grid too large");
   cudaStream_t s = as_stream(stream);
-  const int smem = (2 * kBM * kBK + 2 * bn * kBK) * 2;
-  if (bn == 32) {
-    cudaFuncSetAttribute(gemm_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    gemm_kernel<32><<<grid, 128, smem, s>>>(g);
-  } else if (bn == 64) {
-    cudaFuncSetAttribute(gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    gemm_kernel<64><<<grid, 128, smem, s>>>(g);
-  } else {
-    cudaFuncSetAttribute(gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    gemm_kernel<128><<<grid, 128, smem, s>>>(g);
-  }
-  return check_launch("gemm_kernel");
+  if (bn == 32) return launch_gemm<32>(g, grid, s);
+  if (bn == 64) return launch_gemm<64>(g, grid, s);
+  return launch_gemm<128>(g, grid, s);
 }
 
 extern "C" int64_t fsi_closure_rows_bytes(const fsi_lbm_desc* d) {
@@ -1207,7 +1325,7 @@ extern "C" int fsi_closure_restrict(const fsi_lbm_desc* fine, const float* pops,
 extern "C" int fsi_closure_loss(const float* y, const float* target, const float* b4, int32_t m,
                                 void* dy, void* dyt, int32_t ldt, double* loss, void* stream) {
   FSI_REQUIRE(y && target && b4 && dy && dyt && loss && m > 0 && ldt >= m, "bad loss arguments");
-  closure_loss_kernel<<<grid_for((long long)m * kOutPad, kBlock), kBlock, 0, as_stream(stream)>>>(
+  closure_loss_kernel<<<grid_for(m, kLossRows), kBlock, 0, as_stream(stream)>>>(
       y, target, b4, m, reinterpret_cast<__nv_bfloat16*>(dy), reinterpret_cast<__nv_bfloat16*>(dyt),
       ldt, loss);
   return check_launch("closure_loss_kernel");
@@ -1215,11 +1333,20 @@ extern "C" int fsi_closure_loss(const float* y, const float* target, const float
 
 extern "C" int fsi_closure_colsum(const void* g, int32_t m, int32_t n, float* out, void* stream) {
   FSI_REQUIRE(g && out && m > 0 && n > 0 && n <= 65535, "bad column-sum arguments");
+  cudaStream_t s = as_stream(stream);
+  if (n % 2 == 0 && n <= 2 * kBlock && ((uintptr_t)g & 3) == 0) {
+    ColsumArgs a{};
+    a.g[0] = reinterpret_cast<const __nv_bfloat16*>(g);
+    a.out[0] = out;
+    a.n[0] = n;
+    closure_colsum_kernel<<<dim3(grid_for(m, 128), 1), kBlock, 0, s>>>(a, m);
+    return check_launch("closure_colsum_kernel");
+  }
   int blocks = (int)((m + kBlock - 1) / kBlock);
   if (blocks > 64) blocks = 64;
-  closure_colsum_kernel<<<dim3(blocks, n), kBlock, 0, as_stream(stream)>>>(
+  closure_colsum_any_kernel<<<dim3(blocks, n), kBlock, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(g), m, n, out);
-  return check_launch("closure_colsum_kernel");
+  return check_launch("closure_colsum_any_kernel");
 }
 
 extern "C" int fsi_closure_adam(float* p, const float* g, float* m, float* v, int64_t n, float lr,
@@ -1229,6 +1356,237 @@ extern "C" int fsi_closure_adam(float* p, const float* g, float* m, float* v, in
   closure_adam_kernel<<<grid_for(n, kBlock), kBlock, 0, as_stream(stream)>>>(p, g, m, v, n, lr, beta1,
                                                                               beta2, eps, c1, c2);
   return check_launch("closure_adam_kernel");
+}
+
+namespace fsi {
+namespace {
+
+// Mini-batch rows: xg[i] = x[idx[i]] (BF16 [m][656]), their transpose xt [656][m] and the targets
+// tg[i] = t[idx[i]] ([m][19]). A block moves 64 rows x 64 columns through shared memory, in
+// 16-byte pieces on both sides. m is a multiple of 64.
+constexpr int kPickTile = 64;
+__global__ void __launch_bounds__(kBlock) closure_pick_kernel(const __nv_bfloat16* __restrict__ x,
+                                                              const float* __restrict__ target,
+                                                              const int64_t* __restrict__ idx, int m,
+                                                              __nv_bfloat16* __restrict__ xg,
+                                                              __nv_bfloat16* __restrict__ xt,
+                                                              float* __restrict__ tg) {
+  __shared__ uint16_t tile[kPickTile][kPickTile + 2];
+  __shared__ int64_t rows[kPickTile];
+  const int r0 = blockIdx.x * kPickTile, c0 = blockIdx.y * kPickTile;
+  const int cols = min(kPickTile, kK1 - c0);  // 64, or 16 at the end: whole 16-byte pieces
+  if (threadIdx.x < kPickTile) rows[threadIdx.x] = idx[r0 + threadIdx.x];
+  __syncthreads();
+  for (int i = threadIdx.x; i < kPickTile * (cols / 8); i += kBlock) {
+    const int r = i / (cols / 8), c = (i % (cols / 8)) * 8;
+    const uint4 v = *reinterpret_cast<const uint4*>(x + (size_t)rows[r] * kK1 + c0 + c);
+    *reinterpret_cast<uint4*>(xg + (size_t)(r0 + r) * kK1 + c0 + c) = v;
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      tile[r][c + 2 * j] = (uint16_t)(w[j] & 0xffffu);
+      tile[r][c + 2 * j + 1] = (uint16_t)(w[j] >> 16);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < cols * (kPickTile / 8); i += kBlock) {
+    const int c = i / (kPickTile / 8), r = (i % (kPickTile / 8)) * 8;
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      w[j] = (uint32_t)tile[r + 2 * j][c] | ((uint32_t)tile[r + 2 * j + 1][c] << 16);
+    *reinterpret_cast<uint4*>(xt + (size_t)(c0 + c) * m + r0 + r) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  if (blockIdx.y == 0) {
+    for (int i = threadIdx.x; i < kPickTile * kOut; i += kBlock) {
+      const int r = i / kOut, q = i - r * kOut;
+      tg[(size_t)(r0 + r) * kOut + q] = target[(size_t)rows[r] * kOut + q];
+    }
+  }
+}
+
+// The network's parameters in one float32 array: W1 [64][656], b1, W2 [64][64], b2, W3 [64][64],
+// b3, W4 [32][64], b4 [32].
+constexpr int kH = 64;
+constexpr int kOffB1 = kH * kK1, kOffW2p = kOffB1 + kH, kOffB2 = kOffW2p + kH * kH,
+              kOffW3p = kOffB2 + kH, kOffB3 = kOffW3p + kH * kH, kOffW4p = kOffB3 + kH,
+              kOffB4 = kOffW4p + kOutPad * kH, kParams = kOffB4 + kOutPad;
+
+// Rows per block of a split weight gradient: 64 blocks of 256 rows for 16,384 rows.
+constexpr int kTrainChunk = 256;
+
+struct NetCopies {
+  __nv_bfloat16 *w1, *w2, *w3, *w4, *w2t, *w3t, *w4t;
+  float* bias;
+};
+
+// One Adam step of every parameter (closure_adam_kernel's arithmetic), with the gradients of the
+// zero columns and padding rows cleared, and the BF16 copies of the new weights written.
+__global__ void __launch_bounds__(kBlock) closure_update_kernel(float* __restrict__ p, float* __restrict__ g,
+                                                                float* __restrict__ m, float* __restrict__ v,
+                                                                NetCopies w, float lr, float b1, float b2,
+                                                                float eps, float c1, float c2) {
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= kParams) return;
+  bool unused = false;
+  if (i < kOffB1) {
+    const int c = i % kK1;
+    unused = c >= 27 * kGroup || c % kGroup == kGroup - 1;
+  } else if (i >= kOffW4p) {
+    unused = i < kOffB4 ? (i - kOffW4p) / kH >= kOut : i - kOffB4 >= kOut;
+  }
+  if (unused) g[i] = 0.f;
+  const float gi = unused ? 0.f : g[i];
+  const float mi = b1 * m[i] + (1.f - b1) * gi;
+  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  m[i] = mi;
+  v[i] = vi;
+  const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  p[i] = pi;
+  const __nv_bfloat16 h = __float2bfloat16_rn(pi);
+  if (i < kOffB1) {
+    w.w1[i] = h;
+  } else if (i < kOffW2p) {
+    w.bias[i - kOffB1] = pi;
+  } else if (i < kOffB2) {
+    const int j = i - kOffW2p;
+    w.w2[j] = h;
+    w.w2t[(j % kH) * kH + j / kH] = h;
+  } else if (i < kOffW3p) {
+    w.bias[kH + i - kOffB2] = pi;
+  } else if (i < kOffB3) {
+    const int j = i - kOffW3p;
+    w.w3[j] = h;
+    w.w3t[(j % kH) * kH + j / kH] = h;
+  } else if (i < kOffW4p) {
+    w.bias[2 * kH + i - kOffB3] = pi;
+  } else if (i < kOffB4) {
+    const int j = i - kOffW4p;
+    w.w4[j] = h;
+    w.w4t[(j % kH) * kOutPad + j / kH] = h;
+  } else {
+    w.bias[3 * kH + i - kOffB4] = pi;
+  }
+}
+
+// The buffers of a training step for m rows, carved from one workspace.
+struct TrainWork {
+  __nv_bfloat16 *xg, *xt, *h[3], *ht[3], *dy, *dyt, *dz[3], *dzt[3];
+  float *tg, *z[3], *y;
+};
+
+int64_t carve_train(int64_t m, char* base, TrainWork& w) {
+  int64_t off = 0;
+  auto take = [&](int64_t bytes) {
+    char* p = base ? base + off : nullptr;
+    off += (bytes + 255) & ~(int64_t)255;
+    return p;
+  };
+  auto bf = [&](int64_t n) { return reinterpret_cast<__nv_bfloat16*>(take(2 * n)); };
+  auto f32 = [&](int64_t n) { return reinterpret_cast<float*>(take(4 * n)); };
+  w.xg = bf(m * kK1);
+  w.xt = bf(m * kK1);
+  for (int l = 0; l < 3; ++l) {
+    w.h[l] = bf(m * kH);
+    w.ht[l] = bf(m * kH);
+    w.dz[l] = bf(m * kH);
+    w.dzt[l] = bf(m * kH);
+    w.z[l] = f32(m * kH);
+  }
+  w.dy = bf(m * kOutPad);
+  w.dyt = bf(m * kOutPad);
+  w.y = f32(m * kOutPad);
+  w.tg = f32(m * kOut);
+  return off;
+}
+
+}  // namespace
+}  // namespace fsi
+
+extern "C" int64_t fsi_closure_train_bytes(int32_t m) {
+  if (m <= 0 || m % kBM != 0) {
+    set_error("a training batch has a positive multiple of %d rows, got %d", kBM, m);
+    return -1;
+  }
+  TrainWork w;
+  return carve_train(m, nullptr, w);
+}
+
+extern "C" int fsi_closure_train_step(const fsi_closure_train_desc* d, void* stream) {
+  FSI_REQUIRE(d != nullptr, "NULL descriptor");
+  FSI_REQUIRE(d->x && d->target && d->index && d->params && d->grads && d->adam_m && d->adam_v && d->w1 &&
+                  d->w2 && d->w3 && d->w4 && d->w2t && d->w3t && d->w4t && d->bias && d->work && d->loss &&
+                  d->err,
+              "NULL array");
+  const int64_t need = fsi_closure_train_bytes(d->m);
+  if (need < 0) return FSI_ERR_INVALID_ARG;
+  FSI_REQUIRE(((uintptr_t)d->x & 15) == 0 && ((uintptr_t)d->work & 255) == 0, "x or workspace misaligned");
+  FSI_REQUIRE(d->work_bytes >= need, "workspace of %lld bytes, %lld needed", (long long)d->work_bytes,
+              (long long)need);
+  FSI_REQUIRE(d->step > 0, "the Adam step count starts at 1");
+  FSI_REQUIRE(((uintptr_t)d->grads & 15) == 0, "gradients must be 16-byte aligned");
+  const int m = d->m;
+  cudaStream_t s = as_stream(stream);
+  TrainWork w;
+  carve_train(m, reinterpret_cast<char*>(d->work), w);
+  float* const gr = d->grads;
+  if (cudaMemsetAsync(gr, 0, sizeof(float) * kParams, s) != cudaSuccess ||
+      cudaMemsetAsync(d->loss, 0, sizeof(double), s) != cudaSuccess)
+    return check_launch("memset");
+  closure_pick_kernel<<<dim3(m / kPickTile, (kK1 + kPickTile - 1) / kPickTile), kBlock, 0, s>>>(
+      reinterpret_cast<const __nv_bfloat16*>(d->x), d->target, d->index, m, w.xg, w.xt, w.tg);
+  if (int e = check_launch("closure_pick_kernel")) return e;
+  auto gemm = [&](const void* a, const void* b, int ld, int rows, int cols, int k, int mode, int k_chunk,
+                  float* c, int ldc, const float* bias, __nv_bfloat16* h, __nv_bfloat16* ht, float* zout,
+                  const float* zin) {
+    fsi_closure_gemm_desc q{};
+    q.a = a; q.b = b;
+    q.lda = q.ldb = ld;
+    q.m = rows; q.n = cols; q.k = k; q.k_chunk = k_chunk; q.mode = mode;
+    q.c = c; q.ldc = ldc; q.bias = bias;
+    q.h = h; q.ht = ht; q.ldht = m; q.zout = zout; q.zin = zin; q.err = d->err;
+    return fsi_closure_gemm(&q, stream);
+  };
+  const int kAll = (kK1 + kBK - 1) / kBK * kBK;
+  // forward
+  if (int e = gemm(w.xg, d->w1, kK1, m, kH, kK1, kGeluFwd, kAll, nullptr, 0, d->params + kOffB1, w.h[0],
+                   w.ht[0], w.z[0], nullptr)) return e;
+  if (int e = gemm(w.h[0], d->w2, kH, m, kH, kH, kGeluFwd, kH, nullptr, 0, d->params + kOffB2, w.h[1],
+                   w.ht[1], w.z[1], nullptr)) return e;
+  if (int e = gemm(w.h[1], d->w3, kH, m, kH, kH, kGeluFwd, kH, nullptr, 0, d->params + kOffB3, w.h[2],
+                   w.ht[2], w.z[2], nullptr)) return e;
+  if (int e = gemm(w.h[2], d->w4, kH, m, kOutPad, kH, kStoreF32, kH, w.y, kOutPad, nullptr, nullptr, nullptr,
+                   nullptr, nullptr)) return e;
+  if (int e = fsi_closure_loss(w.y, w.tg, d->params + kOffB4, m, w.dy, w.dyt, m, d->loss, stream)) return e;
+  // backward: dz of each hidden layer from the one above
+  if (int e = gemm(w.dy, d->w4t, kOutPad, m, kH, kOutPad, kGeluBwd, kBK, nullptr, 0, nullptr, w.dz[2],
+                   w.dzt[2], nullptr, w.z[2])) return e;
+  if (int e = gemm(w.dz[2], d->w3t, kH, m, kH, kH, kGeluBwd, kH, nullptr, 0, nullptr, w.dz[1], w.dzt[1],
+                   nullptr, w.z[1])) return e;
+  if (int e = gemm(w.dz[1], d->w2t, kH, m, kH, kH, kGeluBwd, kH, nullptr, 0, nullptr, w.dz[0], w.dzt[0],
+                   nullptr, w.z[0])) return e;
+  // weight gradients: split over the rows so that every SM has a block or two
+  const int chunk = kTrainChunk;
+  if (int e = gemm(w.dyt, w.ht[2], m, kOutPad, kH, m, kAtomicF32, chunk, gr + kOffW4p, kH, nullptr, nullptr,
+                   nullptr, nullptr, nullptr)) return e;
+  if (int e = gemm(w.dzt[2], w.ht[1], m, kH, kH, m, kAtomicF32, chunk, gr + kOffW3p, kH, nullptr, nullptr,
+                   nullptr, nullptr, nullptr)) return e;
+  if (int e = gemm(w.dzt[1], w.ht[0], m, kH, kH, m, kAtomicF32, chunk, gr + kOffW2p, kH, nullptr, nullptr,
+                   nullptr, nullptr, nullptr)) return e;
+  if (int e = gemm(w.dzt[0], w.xt, m, kH, kK1, m, kAtomicF32, 2 * chunk, gr, kK1, nullptr, nullptr, nullptr,
+                   nullptr, nullptr)) return e;
+  ColsumArgs c{};
+  const __nv_bfloat16* src[4] = {w.dz[0], w.dz[1], w.dz[2], w.dy};
+  const int off[4] = {kOffB1, kOffB2, kOffB3, kOffB4}, n[4] = {kH, kH, kH, kOutPad};
+  for (int i = 0; i < 4; ++i) { c.g[i] = src[i]; c.out[i] = gr + off[i]; c.n[i] = n[i]; }
+  closure_colsum_kernel<<<dim3(grid_for(m, 512), 4), kBlock, 0, s>>>(c, m);
+  if (int e = check_launch("closure_colsum_kernel")) return e;
+  auto bf = [](void* p) { return reinterpret_cast<__nv_bfloat16*>(p); };
+  const NetCopies copies{bf(d->w1), bf(d->w2), bf(d->w3), bf(d->w4), bf(d->w2t), bf(d->w3t), bf(d->w4t), d->bias};
+  const float c1 = 1.f - powf(d->beta1, (float)d->step), c2 = 1.f - powf(d->beta2, (float)d->step);
+  closure_update_kernel<<<grid_for(kParams, kBlock), kBlock, 0, s>>>(
+      d->params, gr, d->adam_m, d->adam_v, copies, d->lr, d->beta1, d->beta2, d->eps, c1, c2);
+  return check_launch("closure_update_kernel");
 }
 
 namespace fsi {

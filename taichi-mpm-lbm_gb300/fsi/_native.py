@@ -166,6 +166,22 @@ class ClosureWeights(ctypes.Structure):
     ]
 
 
+class ClosureTrainDesc(ctypes.Structure):
+    _fields_ = [
+        ("x", ctypes.c_void_p), ("target", ctypes.c_void_p), ("index", ctypes.c_void_p),
+        ("params", ctypes.c_void_p), ("grads", ctypes.c_void_p),
+        ("adam_m", ctypes.c_void_p), ("adam_v", ctypes.c_void_p),
+        ("w1", ctypes.c_void_p), ("w2", ctypes.c_void_p), ("w3", ctypes.c_void_p),
+        ("w4", ctypes.c_void_p), ("w2t", ctypes.c_void_p), ("w3t", ctypes.c_void_p),
+        ("w4t", ctypes.c_void_p), ("bias", ctypes.c_void_p),
+        ("work", ctypes.c_void_p), ("work_bytes", ctypes.c_int64),
+        ("loss", ctypes.c_void_p), ("err", ctypes.c_void_p),
+        ("m", ctypes.c_int32), ("step", ctypes.c_int32),
+        ("lr", ctypes.c_float), ("beta1", ctypes.c_float), ("beta2", ctypes.c_float),
+        ("eps", ctypes.c_float),
+    ]
+
+
 GEMM_STORE, GEMM_ATOMIC, GEMM_GELU_FWD, GEMM_GELU_BWD = 0, 1, 2, 3
 BATCH_PARTICLE_ALIGN = 256
 
@@ -229,6 +245,8 @@ _SIGNATURES = {
     "fsi_closure_features": ([ctypes.POINTER(LbmDesc), _VP, _VP, _VP, _VP, ctypes.c_int64, _VP,
                               ctypes.c_int32, ctypes.c_float, ctypes.c_float, _VP, _VP], ctypes.c_int),
     "fsi_closure_gemm": ([ctypes.POINTER(ClosureGemmDesc), _VP], ctypes.c_int),
+    "fsi_closure_train_bytes": ([ctypes.c_int32], ctypes.c_int64),
+    "fsi_closure_train_step": ([ctypes.POINTER(ClosureTrainDesc), _VP], ctypes.c_int),
     "fsi_closure_rows_bytes": ([ctypes.POINTER(LbmDesc)], ctypes.c_int64),
     "fsi_closure_infer_apply": ([ctypes.POINTER(LbmDesc), _VP, _VP, _VP, _VP, ctypes.c_int64,
                                  ctypes.POINTER(ClosureWeights), _VP, _VP, _VP], ctypes.c_int),

@@ -549,20 +549,39 @@ class ClosureTrainer:
     def fit(self, steps: int = 500, batch: int = 16384, lr: float = 2e-3, seed: int = 0,
             halvings: float = 3.0) -> list[float]:
         """Adam on random mini-batches (multiples of 128 rows), the learning rate halving
-        ``halvings`` times over the run; returns the loss history."""
+        ``halvings`` times over the run; returns the loss history. Each step is one call
+        (``fsi_closure_train_step``): the passes of ``ClosureMLP.forward`` / ``backward`` /
+        ``adam_step`` with the rows picked on the device."""
         g = torch.Generator(device="cpu").manual_seed(seed)
         n = self.x.shape[0]
         batch = max(128, min(batch, n) // 128 * 128)
-        hist = []
+        net, dev = self.net, self.x.device
+        x, t = self.x.contiguous(), self.t.contiguous()
+        net.refresh()
+        work = torch.empty(int(nat.load().fsi_closure_train_bytes(batch)), dtype=torch.uint8,
+                           device=dev)
+        loss = torch.zeros(max(steps, 1), dtype=torch.float64, device=dev)
+        d = nat.ClosureTrainDesc()
+        for name, v in (("x", x), ("target", t), ("params", net.params), ("grads", net.grads),
+                        ("adam_m", net.m), ("adam_v", net.v), ("w1", net.w1), ("w2", net.w2),
+                        ("w3", net.w3), ("w4", net.w4), ("w2t", net.w2t), ("w3t", net.w3t),
+                        ("w4t", net.w4t), ("bias", net.bias), ("work", work), ("err", net.err)):
+            setattr(d, name, v.data_ptr())
+        d.work_bytes, d.m = work.numel(), batch
+        d.beta1, d.beta2, d.eps = 0.9, 0.999, 1e-8
+        # Nothing here waits for the device: the next step's rows are drawn while this one runs,
+        # and the losses are read once at the end.
         for it in range(steps):
-            idx = torch.randint(0, n, (batch,), generator=g).to(self.x.device)
-            x = self.x[idx].contiguous()
-            xt = x.t().contiguous()
-            t = self.t[idx].contiguous()
-            y, acts = self.net.forward(x, keep=True)
-            hist.append(self.net.backward(x, y, acts, t, xt=xt))
-            self.net.adam_step(lr=lr * (0.5 ** (it / max(steps, 1) * halvings)))
-        self.net.check()
+            picked = torch.empty(batch, dtype=torch.int64, pin_memory=True)
+            torch.randint(0, n, (batch,), generator=g, out=picked)
+            rows = picked.to(dev, non_blocking=True)
+            net.step_count += 1
+            d.index, d.loss = rows.data_ptr(), loss[it:].data_ptr()
+            d.step = net.step_count
+            d.lr = lr * (0.5 ** (it / max(steps, 1) * halvings))
+            nat.call("fsi_closure_train_step", ctypes.byref(d), nat.stream_ptr())
+        hist = loss[:steps].tolist()
+        net.check()
         return hist
 
 
