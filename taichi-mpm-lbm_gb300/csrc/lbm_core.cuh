@@ -143,6 +143,12 @@ struct Store<FSI_STORAGE_BF16> {
   }
 };
 
+// The 19 storage shifts w_q rho0 by their three values.
+struct Shifts {
+  float w0, w1, w2;
+  __device__ __forceinline__ float operator[](int q) const { return q == 0 ? w0 : (q < 7 ? w1 : w2); }
+};
+
 // Post-stream F_q(x) of a fluid cell in a state of the given parity.
 template <int kStore>
 __device__ __forceinline__ float gather32(const typename Store<kStore>::T* FSI_LAUNCH_RO pops,
@@ -321,23 +327,22 @@ struct StepLanes {
   using V = typename std::conditional<kFast, float2, float>::type;
 };
 
-// Minimum resident 128-thread blocks per SM of the step kernel (caps its registers at
-// 65536 / (128 * n)): scalar exact form by parity, then the packed forms.
-#ifndef FSI_LBM_MIN_BLOCKS_EXACT_EVEN
-#define FSI_LBM_MIN_BLOCKS_EXACT_EVEN 6
-#endif
-#ifndef FSI_LBM_MIN_BLOCKS_EXACT_ODD
-#define FSI_LBM_MIN_BLOCKS_EXACT_ODD 8
-#endif
-#ifndef FSI_LBM_MIN_BLOCKS_FAST
-#define FSI_LBM_MIN_BLOCKS_FAST 6
-#endif
 constexpr int kStepBlock = 128;
 
-template <bool kFast, bool kOdd>
+// Minimum resident 128-thread blocks per SM of the step kernel (caps its registers at
+// 65536 / (128 * n)). From a sweep on the 256^3 channel with spheres, us per step with rho and u
+// read / recomputed:
+//   exact, even   640/610 at 5, 617/610 at 6, 615/608 at 7, 613/595 at 8
+//          odd    672/685 at 6, 644/649 at 7, 624/639 at 8, 607/639 at 9
+//   FP16,  even   443/408 at 4, 394/408 at 5, 363/373 at 6, 361/357 at 7
+//          odd    515/539 at 4, 474/473 at 5, 531/476 at 6, 556/451 at 7
+//   BF16 within 5 % of FP16; fast FP32, even 452/473 at 6 and 472/474 at 5, odd 551/558 at 4,
+//   543/514 at 5, 637/548 at 6.
+template <int kStore, bool kFast, bool kOdd, bool kRecompute>
 constexpr int step_min_blocks() {
-  return kFast ? FSI_LBM_MIN_BLOCKS_FAST
-               : (kOdd ? FSI_LBM_MIN_BLOCKS_EXACT_ODD : FSI_LBM_MIN_BLOCKS_EXACT_EVEN);
+  if (!kFast) return kOdd ? 9 : 8;
+  if (kStore != FSI_STORAGE_F32) return kOdd && !kRecompute ? 5 : 7;
+  return kOdd ? 5 : 6;
 }
 
 // Launch shape of the step kernel: x = z (contiguous), y = groups of `lanes` rows, z = x planes.
@@ -372,21 +377,30 @@ __device__ __forceinline__ void step_cells(const Args& a,
   constexpr int L = StepLanes<kFast>::n;
   using V = typename StepLanes<kFast>::V;
   using Ln = Lanes<V>;
-  Deltas d[L];
   uint32_t fl[L];
   bool live[L];
   bool any = false;
 #pragma unroll
   for (int l = 0; l < L; ++l) {
-    const int o = has[l] ? l : 0;
-    d[l] = Deltas(a.g, ci[o], cj[o], ck[o]);
-    fl[l] = has[l] ? a.flags[d[l].c] : kFlagSolid;
+    fl[l] = has[l] ? a.flags[(uint32_t)((ci[l] * a.g.ny + cj[l]) * a.g.nz + ck[l])] : kFlagSolid;
     live[l] = !(fl[l] & kFlagSolid);
     any = any || live[l];
   }
   if (!any) return;
-  // A solid (or missing) lane reads the cells of a live lane and is never stored.
-  const int src = live[0] ? 0 : L - 1;
+  // A solid (or missing) lane reads the cells of the live lane and is never stored. It takes that
+  // lane's coordinates here, before anything is derived from them: picked by an index chosen at
+  // run time, the neighbour offsets would live in local memory.
+  int i[L], j[L], k[L];
+#pragma unroll
+  for (int l = 0; l < L; ++l) { i[l] = ci[l]; j[l] = cj[l]; k[l] = ck[l]; }
+  if constexpr (L == 2) {
+    const uint32_t f0 = fl[0];
+    if (!live[0]) { fl[0] = fl[1]; i[0] = ci[1]; j[0] = cj[1]; k[0] = ck[1]; }
+    if (!live[1]) { fl[1] = f0; i[1] = ci[0]; j[1] = cj[0]; k[1] = ck[0]; }
+  }
+  Deltas d[L];
+#pragma unroll
+  for (int l = 0; l < L; ++l) d[l] = Deltas(a.g, i[l], j[l], k[l]);
   const uint32_t n = (uint32_t)a.g.n;
   typename St::T* __restrict__ pops = reinterpret_cast<typename St::T*>(a.pops);
 
@@ -396,10 +410,9 @@ __device__ __forceinline__ void step_cells(const Args& a,
     uint32_t sl[L];
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-      const int ll = live[l] ? l : src;
       // F_q(x) = f*_q(x - e_q) in slot opp(q) there, or f*_opp(q)(x) in slot q here when
       // x - e_q is solid (half-way bounce-back).
-      sl[l] = (!kOdd || q == 0) ? q * n + d[ll].c : odd_src(d[ll], fl[ll], q, n);
+      sl[l] = (!kOdd || q == 0) ? q * n + d[l].c : odd_src(d[l], fl[l], q, n);
     }
     if constexpr (L == 2) {
       F[q] = St::ld2(pops, sl[0], sl[1], a.shift[q]);
@@ -413,7 +426,7 @@ __device__ __forceinline__ void step_cells(const Args& a,
 
   uint32_t c[L];
 #pragma unroll
-  for (int l = 0; l < L; ++l) c[l] = d[live[l] ? l : src].c;
+  for (int l = 0; l < L; ++l) c[l] = d[l].c;
   V gx, gy, gz, rho, ux, uy, uz;
 #pragma unroll
   for (int l = 0; l < L; ++l) {
@@ -450,6 +463,19 @@ __device__ __forceinline__ void step_cells(const Args& a,
   if (kFast) mrt_collide_fast(F, rho, ux, uy, uz, gx, gy, gz, a.s, out);
   else collide_cell(mF, ux, uy, uz, gx, gy, gz, a.s, a.sg, out);
 
+  // The stores address what the loads did. Seen as the same expressions, up to 19 64-bit
+  // addresses per lane and the neighbour offsets would be kept from one to the other across the
+  // collision, in registers that the loads in flight need; coordinates that only now become
+  // known make them again. (Exact form at 256^3: even steps 641 -> 608 us, 771 -> 615 with rho and
+  // u read. Its odd step with rho and u recomputed is short of issue slots instead: 639 us as it
+  // is, 647 with the offsets made again.)
+  if constexpr (kFast || !kOdd || !kRecompute) {
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+      asm volatile("" : "+r"(j[l]), "+r"(k[l]));
+      d[l] = Deltas(a.g, i[l], j[l], k[l]);
+    }
+  }
 #pragma unroll
   for (int q = 0; q < 19; ++q) {
     // f*_q goes to slot opp(q) of this cell (even step, or odd-step bounce-back) or to slot q
@@ -471,7 +497,7 @@ __device__ __forceinline__ void step_cells(const Args& a,
 }
 
 template <int kStore, bool kFast, bool kOdd, bool kRecompute>
-__global__ void __launch_bounds__(kStepBlock, (step_min_blocks<kFast, kOdd>()))
+__global__ void __launch_bounds__(kStepBlock, (step_min_blocks<kStore, kFast, kOdd, kRecompute>()))
     lbm_step_kernel(StepArgs a) {
   constexpr int L = StepLanes<kFast>::n;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
