@@ -36,7 +36,7 @@ struct fsi_batch {
   int variant = 1;
   fsi::BatchSolid* sol = nullptr;   // device
   fsi::Tile* ptiles = nullptr;      // device: (scene, particle block of kBlock particles)
-  fsi::Tile* ctiles = nullptr;      // device: (scene, first node block of 8)
+  fsi::Tile* ctiles = nullptr;      // device: (scene, first node block of kBlock)
   int nptiles = 0;
   int nctiles = 0;
   long long capacity = 0;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock)
                         t.first * kBlock + threadIdx.x, sm);
 }
 
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 1024 / kBlock)
     batch_g2p_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
                      const Tile* __restrict__ ptiles, PView P, const float4* grid_all) {
   const Tile t = ptiles[blockIdx.x];
@@ -205,17 +205,20 @@ __global__ void __launch_bounds__(kBlock)
   g2p_body(m, P, grid_all + lat[t.lattice].off, t.first * kBlock + threadIdx.x);
 }
 
-// One warp per node block: CTA (scene, first block) covers kBlock / 32 blocks.
+// CTA (scene, first block) covers kBlock node blocks, a warp 32 of them. (With a warp per block,
+// 47 us for 64 scenes: 320,000 warps to find the few dirty blocks.)
 __global__ void __launch_bounds__(kBlock)
     batch_clear_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
                        const Tile* __restrict__ ctiles, float4* grid_all, uint8_t* dirty_all) {
   const Tile t = ctiles[blockIdx.x];
   const Mpm m = sol[t.lattice].m;
-  clear_body(m, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
-             (long long)t.first + (threadIdx.x >> 5));
+  clear_dirty_body(m, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
+                   t.first + (threadIdx.x & ~31));
 }
 
-__global__ void __launch_bounds__(kBlock)
+// Three blocks per SM: 187 us for 64 scenes, against 212 at its natural 101 registers (two) and 210
+// at 64 (four, spills).
+__global__ void __launch_bounds__(kBlock, 3)
     batch_coupling_forces_kernel(const BatchLattice* __restrict__ lat,
                                  const BatchSolid* __restrict__ sol, const Tile* __restrict__ ptiles,
                                  ForceArgs base, float dt_ratio, int build_fraction) {
@@ -243,6 +246,40 @@ int check_solids(const fsi_batch* b) {
 }  // namespace fsi
 
 using namespace fsi;
+
+namespace {
+// Cuts the lattices into step tiles of step_tile_cells cells (for the fast forms, of half as many
+// pairs of cells: step_unit).
+int set_step_tiles(fsi_batch* b, int step_tile_cells) {
+  const int lanes = b->arithmetic == FSI_ARITH_FAST ? 2 : 1;
+  std::vector<Tile> tiles;
+  for (int s = 0; s < b->count; ++s)
+    for (long long c = 0; c < step_units(b->host[s].g, lanes); c += step_tile_cells / lanes)
+      tiles.push_back(Tile{s, (int)c});
+  Tile* dev = nullptr;
+  if (cudaMalloc(&dev, sizeof(Tile) * tiles.size()) != cudaSuccess ||
+      cudaMemcpy(dev, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice) !=
+          cudaSuccess) {
+    cudaFree(dev);
+    const int e = check_launch("batch step tiles");
+    return e ? e : FSI_ERR_CUDA;
+  }
+  if (b->step_tiles != b->tiles) cudaFree(b->step_tiles);
+  b->step_tiles = dev;
+  b->nstep_tiles = (int)tiles.size();
+  b->step_tile_cells = step_tile_cells;
+  return FSI_OK;
+}
+
+// A block's start (tile, lattice table, rates) costs less the more cells it takes: 64 scenes, FP16,
+// 0.637 ms per step with 256 cells, 0.600 with 512, 0.594 with 1,024. Larger tiles are the
+// default as long as they still make four waves of six blocks on 152 SMs.
+int default_step_tiles(fsi_batch* b) {
+  for (const int cells : {1024, 512})
+    if (b->cells / cells >= 4ll * 6 * 152) return set_step_tiles(b, cells);
+  return set_step_tiles(b, kTileCells);
+}
+}  // namespace
 
 extern "C" int fsi_batch_create(const fsi_batch_lattice* lattices, int32_t count, int32_t storage,
                                 int32_t arithmetic, fsi_batch** out) {
@@ -304,6 +341,10 @@ extern "C" int fsi_batch_create(const fsi_batch_lattice* lattices, int32_t count
   b->step_tiles = b->tiles;
   b->nstep_tiles = b->ntiles;
   b->step_tile_cells = kTileCells;
+  if (const int e = default_step_tiles(b)) {
+    fsi_batch_destroy(b);
+    return e;
+  }
   *out = b;
   return FSI_OK;
 }
@@ -376,20 +417,7 @@ extern "C" int fsi_batch_tune(fsi_batch* b, int32_t step_tile_cells, int32_t var
               "step tile of %d cells is not a multiple of %d (at most 8192)", step_tile_cells,
               kStepBlock * lanes);
   FSI_REQUIRE(variant >= 0 && variant <= 2, "unknown variant %d", variant);
-  std::vector<Tile> tiles;
-  for (int s = 0; s < b->count; ++s)
-    for (long long c = 0; c < b->host[s].g.n; c += step_tile_cells) tiles.push_back(Tile{s, (int)c});
-  Tile* dev = nullptr;
-  if (cudaMalloc(&dev, sizeof(Tile) * tiles.size()) != cudaSuccess ||
-      cudaMemcpy(dev, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice) !=
-          cudaSuccess) {
-    cudaFree(dev);
-    return check_launch("fsi_batch_tune");
-  }
-  if (b->step_tiles != b->tiles) cudaFree(b->step_tiles);
-  b->step_tiles = dev;
-  b->nstep_tiles = (int)tiles.size();
-  b->step_tile_cells = step_tile_cells;
+  if (int e = set_step_tiles(b, step_tile_cells)) return e;
   b->variant = variant;
   return FSI_OK;
 }
@@ -463,7 +491,7 @@ extern "C" int fsi_batch_set_solids(fsi_batch* b, const fsi_batch_solid* solids,
     for (long long p = in.particle_offset; p < S.m.n; p += kBlock)
       ptiles.push_back(Tile{s, (int)(p / kBlock)});
     const long long nb = (long long)S.m.nbx * S.m.nby * S.m.nbz;
-    for (long long q = 0; q < nb; q += kBlock / 32) ctiles.push_back(Tile{s, (int)q});
+    for (long long q = 0; q < nb; q += kBlock) ctiles.push_back(Tile{s, (int)q});
     block_off += nb;
     next = S.m.n;
   }

@@ -57,24 +57,19 @@ __device__ __forceinline__ bool grid_barrier(const PersistArgs& a, unsigned& epo
 template <int kStore, bool kFast, bool kOdd>
 __device__ __forceinline__ void persist_step_tiles(const PersistArgs& a, float* force) {
   constexpr int NL = StepLanes<kFast>::n;
+  __shared__ Rates rates;
   for (int ti = blockIdx.x; ti < a.nstep_tiles; ti += gridDim.x) {
     const Tile t = a.step_tiles[ti];
     const BatchLattice& L = a.lat[t.lattice];
-    const LatticeView v = view_of<kStore>(L, a.pops, a.macro, force, nullptr, a.flags);
-    const int n = (int)L.g.n;
-    for (int base = 0; base < a.step_tile_cells; base += kBlock * NL) {
+    __syncthreads();  // the previous tile's rates are no longer read
+    load_rates(L, rates);
+    __syncthreads();
+    const LatticeView v = view_of<kStore>(L, rates, a.pops, a.macro, force, nullptr, a.flags);
+    for (int off = threadIdx.x; off < a.step_tile_cells / NL; off += kBlock) {
       int ci[NL], cj[NL], ck[NL];
       bool has[NL];
-      bool any = false;
-#pragma unroll
-      for (int l = 0; l < NL; ++l) {
-        const int off = base + threadIdx.x + l * kBlock;
-        const int c = t.first + off;
-        has[l] = off < a.step_tile_cells && c < n;
-        any = any || has[l];
-        cell_ijk(L.g, has[l] ? c : t.first, ci[l], cj[l], ck[l]);
-      }
-      if (any) step_cells<kStore, kFast, kOdd, false, LatticeView>(v, ci, cj, ck, has);
+      if (step_unit<NL>(L.g, (long long)t.first + off, ci, cj, ck, has))
+        step_cells<kStore, kFast, kOdd, false, LatticeView>(v, ci, cj, ck, has);
     }
   }
 }
@@ -151,8 +146,8 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
       for (int ti = blockIdx.x; ti < a.nctiles; ti += gridDim.x) {
         const Tile t = a.ctiles[ti];
         const BatchSolid& S = a.sol[t.lattice];
-        clear_body(S.m, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
-                   (long long)t.first + (threadIdx.x >> 5));
+        clear_dirty_body(S.m, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
+                         t.first + (threadIdx.x & ~31));
       }
       // the next substep's unsupported / partial / clipped counts start from zero
       if (blockIdx.x == 0 && sub + 1 < a.substeps)

@@ -17,35 +17,35 @@ struct BatchStepArgs {
   const uint32_t* flags;
 };
 
-// Minimum resident blocks per SM of register-cap variant kVar (0..2).
-template <bool kFast, bool kOdd, int kVar>
+// Minimum resident blocks per SM of register-cap variant kVar (0..2), 1 being the default.
+// Measured on 64 scenes with tiles of 1,024 cells, us per step, by blocks. FP16, even: 606 at 4,
+// 570 at 6, 572 at 8 (rho and u read); odd: 650 at 4, 851 at 5, 967 at 6 (spills), and with rho and
+// u recomputed 669, 649, 740. FP32 exact, even: 906 at 4, 928 at 6, 808 at 8; odd: 927 at 6, 903 at 8.
+template <bool kFast, bool kOdd, bool kRecompute, int kVar>
 constexpr int batch_min_blocks() {
-  return (kFast || !kOdd) ? (kVar == 0 ? 4 : kVar == 1 ? 6 : 8) : (kVar == 0 ? 6 : 8);
+  if (kFast && kOdd) return kVar == 0 ? 4 : kVar == 1 ? (kRecompute ? 5 : 4) : 6;
+  if (kFast) return kVar == 0 ? 4 : kVar == 1 ? 6 : 8;
+  return !kOdd ? (kVar == 0 ? 4 : kVar == 1 ? 8 : 6) : (kVar == 0 ? 6 : 8);
 }
 
 // kStepBlock threads cover a tile of reps * kStepBlock * lanes cells: the exact form takes
 // one cell per thread and pass, the fast forms two (the packed lanes).
 template <int kStore, bool kFast, bool kOdd, bool kRecompute, int kVar>
-__global__ void __launch_bounds__(kStepBlock, (batch_min_blocks<kFast, kOdd, kVar>()))
+__global__ void __launch_bounds__(kStepBlock, (batch_min_blocks<kFast, kOdd, kRecompute, kVar>()))
     batch_step_kernel(BatchStepArgs b) {
   constexpr int NL = StepLanes<kFast>::n;
   const int kReps = b.reps;
   const Tile t = b.tiles[blockIdx.x];
   const BatchLattice& L = b.lat[t.lattice];
-  const LatticeView v = view_of<kStore>(L, b.pops, b.macro, b.force, b.force_prev, b.flags);
-  const int n = (int)L.g.n;
+  __shared__ Rates rates;
+  load_rates(L, rates);
+  __syncthreads();
+  const LatticeView v = view_of<kStore>(L, rates, b.pops, b.macro, b.force, b.force_prev, b.flags);
   for (int r = 0; r < kReps; ++r) {
     int ci[NL], cj[NL], ck[NL];
     bool has[NL];
-    bool any = false;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      const int c = t.first + threadIdx.x + (r * NL + l) * kStepBlock;
-      has[l] = c < n;
-      any = any || has[l];
-      cell_ijk(L.g, has[l] ? c : t.first, ci[l], cj[l], ck[l]);
-    }
-    if (any) step_cells<kStore, kFast, kOdd, kRecompute, LatticeView>(v, ci, cj, ck, has);
+    if (step_unit<NL>(L.g, (long long)t.first + r * kStepBlock + threadIdx.x, ci, cj, ck, has))
+      step_cells<kStore, kFast, kOdd, kRecompute, LatticeView>(v, ci, cj, ck, has);
   }
 }
 

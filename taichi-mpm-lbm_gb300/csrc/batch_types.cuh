@@ -27,7 +27,7 @@ struct BatchLattice {
 
 struct Tile {
   int lattice;
-  int first;  // first cell (lattice tiles), particle block or node block (solid tiles)
+  int first;  // first cell (lattice tiles), step unit, particle block or node block (solid tiles)
 };
 
 struct BatchSolid {
@@ -44,6 +44,28 @@ __device__ __forceinline__ void cell_ijk(const LbmGeom& g, int c, int& i, int& j
   k = r - j * g.nz;
 }
 
+// The units of a lattice's step: cells, or for the fast forms the pairs of cells (i, j, k) and
+// (i, j + 1, k), j even, which share all neighbour offsets but those along y (two cells that
+// share none spill: the odd step of 64 FP16 scenes took 1,004 us with pairs 128 cells apart).
+__host__ __device__ inline long long step_units(const LbmGeom& g, int lanes) {
+  return (long long)g.nx * ((g.ny + lanes - 1) / lanes) * g.nz;
+}
+// The cells of unit u (clamped to unit 0 past the end, has[] false).
+template <int L>
+__device__ __forceinline__ bool step_unit(const LbmGeom& g, long long u, int (&ci)[L], int (&cj)[L],
+                                          int (&ck)[L], bool (&has)[L]) {
+  const int rows = (g.ny + L - 1) / L;
+  const bool in = u < (long long)g.nx * rows * g.nz;
+  const int v = in ? (int)u : 0;
+  const int i = v / (rows * g.nz), r = v - i * rows * g.nz, j = L * (r / g.nz), k = r - (r / g.nz) * g.nz;
+#pragma unroll
+  for (int l = 0; l < L; ++l) {
+    ci[l] = i; cj[l] = j + l; ck[l] = k;
+    has[l] = in && j + l < g.ny;
+  }
+  return in;
+}
+
 // The lattice of a tile as the argument type of step_cells.
 struct LatticeView {
   LbmGeom g;
@@ -54,12 +76,27 @@ struct LatticeView {
   const uint32_t* __restrict__ flags;
   const float* s;
   const float* sg;
-  const float* shift;
+  Shifts shift;
   int write_faces;
 };
 
+__device__ __forceinline__ Shifts shifts_of(const BatchLattice& L) {
+  return Shifts{L.shift[0], L.shift[1], L.shift[7]};
+}
+
+// The relaxation rates of a block's lattice in shared memory. Read from the table in global
+// memory, the 19 or 38 of them were as many loads per thread again as its populations.
+struct Rates {
+  float s[19], sg[19];
+};
+__device__ __forceinline__ void load_rates(const BatchLattice& L, Rates& r) {
+  if (threadIdx.x < 19) r.s[threadIdx.x] = L.s[threadIdx.x];
+  else if (threadIdx.x >= 32 && threadIdx.x < 32 + 19) r.sg[threadIdx.x - 32] = L.sg[threadIdx.x - 32];
+}
+
 template <int kStore>
-__device__ __forceinline__ LatticeView view_of(const BatchLattice& L, void* pops, float* macro,
+__device__ __forceinline__ LatticeView view_of(const BatchLattice& L, const Rates& rates,
+                                               void* pops, float* macro,
                                                const float* force, const float* force_prev,
                                                const uint32_t* flags) {
   using T = typename Store<kStore>::T;
@@ -70,9 +107,9 @@ __device__ __forceinline__ LatticeView view_of(const BatchLattice& L, void* pops
   v.force = force + 3 * L.off;
   v.force_prev = force_prev ? force_prev + 3 * L.off : nullptr;
   v.flags = flags + L.off;
-  v.s = L.s;
-  v.sg = L.sg;
-  v.shift = L.shift;
+  v.s = rates.s;
+  v.sg = rates.sg;
+  v.shift = shifts_of(L);
   v.write_faces = 0;
   return v;
 }
@@ -99,9 +136,10 @@ __device__ __forceinline__ void batch_macro_cell(const BatchLattice& L, int c, c
   const uint32_t n = (uint32_t)L.g.n;
   const auto* pops = reinterpret_cast<const typename Store<kStore>::T*>(pops_v) + 19 * L.off;
   const float* force = force_all + 3 * L.off;
+  const Shifts shift = shifts_of(L);
   float F[19];
 #pragma unroll
-  for (int q = 0; q < 19; ++q) F[q] = gather32<kStore>(pops, n, d, fl, q, parity, L.shift[q]);
+  for (int q = 0; q < 19; ++q) F[q] = gather32<kStore>(pops, n, d, fl, q, parity, shift[q]);
   float rho, ux, uy, uz;
   macro_any<kFast>(F, force[c], force[n + c], force[2 * n + c], rho, ux, uy, uz);
   macro[c] = make_float4(ux, uy, uz, rho);
@@ -156,7 +194,7 @@ struct PersistArgs {
   int step_tile_cells;
   const Tile* ptiles;  // kBlock particles of one scene each
   int nptiles;
-  const Tile* ctiles;  // kBlock / 32 node blocks of one scene each
+  const Tile* ctiles;  // kBlock node blocks of one scene each
   int nctiles;
   int count;
   PView P;

@@ -105,36 +105,10 @@ struct G2P {
   }
 };
 
-__global__ void __launch_bounds__(kBlock) clear_kernel(Mpm m, float4* __restrict__ grid,
-                                                       uint8_t* __restrict__ dirty) {
-  clear_body(m, grid, dirty, ((long long)blockIdx.x * kBlock + threadIdx.x) >> 5);
-}
-
-// Zeroes the dirty 4^3 node blocks: each warp reads the flags of 32 consecutive blocks with
-// one load, then zeroes the dirty ones together (two nodes per lane) and resets their flags.
-// Launches one warp per 32 blocks instead of one per block.
+// One warp per 32 node blocks.
 __global__ void __launch_bounds__(kBlock) clear_dirty_kernel(Mpm m, float4* __restrict__ grid,
                                                              uint8_t* __restrict__ dirty) {
-  const long long nblocks = (long long)m.nbx * m.nby * m.nbz;
-  const int lane = threadIdx.x & 31;
-  const long long b0 = (((long long)blockIdx.x * kBlock + threadIdx.x) >> 5) << 5;
-  const long long mine = b0 + lane;
-  const bool d = mine < nblocks && dirty[mine] != 0;
-  unsigned todo = __ballot_sync(0xffffffffu, d);
-  while (todo) {
-    const int l = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const long long b = b0 + l;
-    const int bi = (int)(b / ((long long)m.nby * m.nbz));
-    const int bj = (int)((b / m.nbz) % m.nby);
-    const int bk = (int)(b % m.nbz);
-#pragma unroll
-    for (int t = lane; t < 64; t += 32) {
-      const int i = bi * 4 + (t >> 4), j = bj * 4 + ((t >> 2) & 3), k = bk * 4 + (t & 3);
-      if (i < m.nx && j < m.ny && k < m.nz) grid[node_index(m, i, j, k)] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  if (d) dirty[mine] = 0;
+  clear_dirty_body(m, grid, dirty, (((long long)blockIdx.x * kBlock + threadIdx.x) >> 5) << 5);
 }
 
 __global__ void polar_kernel(const float* __restrict__ F, float* __restrict__ R, long long n) {
@@ -378,8 +352,8 @@ extern "C" int fsi_mpm_substep_noalloc(const fsi_mpm_desc* d, const fsi_particle
     return check_launch("no-alloc scratch clear");
   if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel (no-alloc)", m, P, g4, dirty)) return e;
   if (int e = launch_tiled<G2P>(m.threads, m, s, "g2p_kernel (no-alloc)", m, P, (const float4*)g4)) return e;
-  clear_kernel<<<grid_for(nblocks * 32, kBlock), kBlock, 0, s>>>(m, g4, dirty);
-  return check_launch("clear_kernel (no-alloc)");
+  clear_dirty_kernel<<<grid_for(nblocks, kBlock), kBlock, 0, s>>>(m, g4, dirty);
+  return check_launch("clear_dirty_kernel (no-alloc)");
 }
 
 extern "C" int fsi_coupled_substep_tiled(const fsi_coupling_desc* c, const fsi_mpm_desc* d,

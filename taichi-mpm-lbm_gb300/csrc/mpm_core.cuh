@@ -849,24 +849,30 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
   }
 }
 
-// Zero every dirty 4^3 node block and reset its flag (one warp per block).
-// Clears node block b when dirty (one warp per block; the warp's lanes all call it).
-__device__ __forceinline__ void clear_body(const Mpm& m, float4* __restrict__ grid,
-                                           uint8_t* __restrict__ dirty, long long b) {
+// Zeroes the dirty ones of the 32 4^3 node blocks from b0 (one warp; its lanes all call it): the
+// flags in one load, then two nodes per lane of each dirty block, and the flags reset.
+__device__ __forceinline__ void clear_dirty_body(const Mpm& m, float4* __restrict__ grid,
+                                                 uint8_t* __restrict__ dirty, long long b0) {
   const long long nblocks = (long long)m.nbx * m.nby * m.nbz;
-  if (b >= nblocks || dirty[b] == 0) return;
   const int lane = threadIdx.x & 31;
-  const int bi = (int)(b / ((long long)m.nby * m.nbz));
-  const int bj = (int)((b / m.nbz) % m.nby);
-  const int bk = (int)(b % m.nbz);
-  for (int t = lane; t < 64; t += 32) {
-    const int i = bi * 4 + (t >> 4), j = bj * 4 + ((t >> 2) & 3), k = bk * 4 + (t & 3);
-    if (i < m.nx && j < m.ny && k < m.nz) grid[node_index(m, i, j, k)] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const long long mine = b0 + lane;
+  const bool d = mine < nblocks && dirty[mine] != 0;
+  unsigned todo = __ballot_sync(0xffffffffu, d);
+  while (todo) {
+    const int l = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const long long b = b0 + l;
+    const int bi = (int)(b / ((long long)m.nby * m.nbz));
+    const int bj = (int)((b / m.nbz) % m.nby);
+    const int bk = (int)(b % m.nbz);
+#pragma unroll
+    for (int t = lane; t < 64; t += 32) {
+      const int i = bi * 4 + (t >> 4), j = bj * 4 + ((t >> 2) & 3), k = bk * 4 + (t & 3);
+      if (i < m.nx && j < m.ny && k < m.nz) grid[node_index(m, i, j, k)] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
-  __syncwarp();
-  if (lane == 0) dirty[b] = 0;
+  if (d) dirty[mine] = 0;
 }
-
 
 // Host-side validation of a solver descriptor and its particle arrays.
 int make_mpm(const fsi_mpm_desc* d, const fsi_particles* p, Mpm& m, PView& v) {

@@ -73,7 +73,10 @@ class LatticeBatch:
         self._fcur = 0
         self._fprev = -1
         self._initialized = False
-        self.tuning = {"step_tile_cells": 256, "variant": 1}
+        # the library's choice until fsi.autotune.tune_lattice_batch makes another: the largest
+        # step tile that still gives four waves of blocks
+        tile = next((t for t in (1024, 512) if n // t >= 4 * 6 * 152), 256)
+        self.tuning = {"step_tile_cells": tile, "variant": 1}
 
     # ------------------------------------------------------------ state / tuning
     def snapshot(self) -> dict:
