@@ -558,8 +558,12 @@ __device__ __forceinline__ void p2g_runs_body(const Mpm& m, const PView& P, floa
     return;
   }
   if (!in) return;
+  // Odd lanes walk the stencil backwards: the two particles of a sub-cell pair, which share a base
+  // cell, then add into different nodes at each step.
+  const bool rev = (threadIdx.x & 1) != 0;
 #pragma unroll 1
-  for (int s = 0; s < 27; ++s) {
+  for (int t = 0; t < 27; ++t) {
+    const int s = rev ? 26 - t : t;
     const int oi = s / 9, oj = (s / 3) % 3, ok = s % 3;
     const int i = base[0] + oi, j = base[1] + oj, k = base[2] + ok;
     if (!inside(m, i, j, k)) continue;
