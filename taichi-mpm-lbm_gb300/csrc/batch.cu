@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock)
                         t.first * kBlock + threadIdx.x, sm);
 }
 
-__global__ void __launch_bounds__(kBlock, 1024 / kBlock)
+__global__ void __launch_bounds__(kBlock, 1280 / kBlock)
     batch_g2p_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
                      const Tile* __restrict__ ptiles, PView P, const float4* grid_all) {
   const Tile t = ptiles[blockIdx.x];
@@ -205,15 +205,16 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock)
   g2p_body(m, P, grid_all + lat[t.lattice].off, t.first * kBlock + threadIdx.x);
 }
 
-// CTA (scene, first block) covers kBlock node blocks, a warp 32 of them. (With a warp per block,
-// 47 us for 64 scenes: 320,000 warps to find the few dirty blocks.)
+// CTA (scene, first block) covers kBlock node blocks and works on the dirty ones together: 7 us for
+// 64 scenes, against 14 with a warp for 32 blocks and 47 with a warp per block.
 __global__ void __launch_bounds__(kBlock)
     batch_clear_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
                        const Tile* __restrict__ ctiles, float4* grid_all, uint8_t* dirty_all) {
   const Tile t = ctiles[blockIdx.x];
   const Mpm m = sol[t.lattice].m;
+  __shared__ DirtyList l;
   clear_dirty_body(m, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
-                   t.first + (threadIdx.x & ~31));
+                   t.first + (int)threadIdx.x, l);
 }
 
 // Three blocks per SM: 187 us for 64 scenes, against 212 at its natural 101 registers (two) and 210

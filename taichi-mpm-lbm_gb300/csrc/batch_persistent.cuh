@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
   extern __shared__ float4 persist_smem[];
   float (*tile)[kTileCap] = reinterpret_cast<float (*)[kTileCap]>(persist_smem);
   auto& p2g_smem = *reinterpret_cast<ScatterSmem<kBlock>*>(persist_smem);
+  auto& dirty_list = *reinterpret_cast<DirtyList*>(persist_smem);
   unsigned epoch = 0;
   int prev = a.prev;
   int* const words = reinterpret_cast<int*>(a.fa.cnt);  // [count][12] counter words
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
         const Tile t = a.ctiles[ti];
         const BatchSolid& S = a.sol[t.lattice];
         clear_dirty_body(S.m, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
-                         t.first + (threadIdx.x & ~31));
+                         t.first + (int)threadIdx.x, dirty_list);
       }
       // the next substep's unsupported / partial / clipped counts start from zero
       if (blockIdx.x == 0 && sub + 1 < a.substeps)

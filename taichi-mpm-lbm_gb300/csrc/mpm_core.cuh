@@ -194,6 +194,22 @@ struct Box {
   int vol;
 };
 
+// The part in the grid of the box [sh[0..2], sh[3..5]]; vol: its nodes, at most kTileCap + 1.
+__device__ __forceinline__ Box box_of(const Mpm& m, const int* sh) {
+  Box box;
+  const int n[3] = {m.nx, m.ny, m.nz};
+  long long vol = 1;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int lo = max(sh[a], 0), hi = min(sh[3 + a], n[a] - 1);
+    box.lo[a] = lo;
+    box.ext[a] = hi >= lo ? hi - lo + 1 : 0;
+    vol *= box.ext[a];
+  }
+  box.vol = vol > (long long)kTileCap ? kTileCap + 1 : (int)vol;
+  return box;
+}
+
 __device__ bool cta_box(const Mpm& m, bool act, const int base[3], Box& box, int* sh) {
   // sh: 6 ints of shared scratch
   if (threadIdx.x < 3) { sh[threadIdx.x] = 0x7fffffff; sh[3 + threadIdx.x] = -0x7fffffff; }
@@ -208,17 +224,61 @@ __device__ bool cta_box(const Mpm& m, bool act, const int base[3], Box& box, int
   }
   __syncthreads();
   if (sh[0] == 0x7fffffff) return false;  // no active particle
-  const int n[3] = {m.nx, m.ny, m.nz};
-  long long vol = 1;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    int lo = max(sh[a], 0), hi = min(sh[3 + a], n[a] - 1);
-    box.lo[a] = lo;
-    box.ext[a] = hi >= lo ? hi - lo + 1 : 0;
-    vol *= box.ext[a];
-  }
-  box.vol = vol > (long long)kTileCap ? kTileCap + 1 : (int)vol;
+  box = box_of(m, sh);
   return true;
+}
+
+// For a CTA whose box is too large, the usual reason being that its particles end one body and
+// begin the next: cuts it in two where consecutive particles are farthest apart. Returns this
+// thread's part (false: before the cut) and both boxes; every thread calls it.
+// sh: 13 ints of shared scratch, last: 4 ints per warp.
+__device__ bool cut_boxes(const Mpm& m, bool act, const int base[3], Box box[2], int* sh, int (*last)[4]) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  __syncthreads();  // the whole box's scratch is no longer read
+  if (t < 12) sh[t] = t % 6 < 3 ? 0x7fffffff : -0x7fffffff;
+  if (t == 12) sh[12] = 0;
+  if (lane == 31) {
+    last[warp][0] = base[0]; last[warp][1] = base[1]; last[warp][2] = base[2]; last[warp][3] = act;
+  }
+  __syncthreads();
+  int before[4] = {base[0], base[1], base[2], act};
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    before[a] = __shfl_up_sync(0xffffffffu, before[a], 1);
+    if (lane == 0 && warp > 0) before[a] = last[warp - 1][a];
+  }
+  int far = 0;  // distance << 10 | thread
+  if (act && t > 0 && before[3]) {
+    // each term below 2^20, whatever the coordinates
+    unsigned d = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const unsigned u = base[a] > before[a] ? (unsigned)base[a] - (unsigned)before[a]
+                                             : (unsigned)before[a] - (unsigned)base[a];
+      d += min(u, 0x7ffffu);
+    }
+    far = (int)(min(d, 0x1fffffu) << 10) | t;
+  }
+  far = __reduce_max_sync(0xffffffffu, far);
+  if (lane == 0) atomicMax(&sh[12], far);
+  __syncthreads();
+  const bool part = t >= (sh[12] & 1023);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const bool mine = act && part == (h == 1);
+      const int lo = __reduce_min_sync(0xffffffffu, mine ? base[a] : 0x7fffffff);
+      const int hi = __reduce_max_sync(0xffffffffu, mine ? base[a] + 2 : -0x7fffffff);
+      if (lane == 0) { atomicMin(&sh[6 * h + a], lo); atomicMax(&sh[6 * h + 3 + a], hi); }
+    }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    box[h] = box_of(m, sh + 6 * h);
+    if (sh[6 * h] == 0x7fffffff) box[h].vol = 0;
+  }
+  return part;
 }
 
 __device__ __forceinline__ void load_particle_x(const PView& P, long long cap, int p, float x[3]) {
@@ -758,59 +818,27 @@ __device__ __forceinline__ void grid_op(const Mpm& m, float4 node, int i, int j,
   }
 }
 
-// Grid update + G2P of particle p (this thread) within its CTA; every thread calls it.
-// kExtTile: the tile is the caller's shared memory `ext` (3 x kTileCap floats) instead of a
-// static array of its own.
-template <bool kExtTile = false>
-__device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
-                                         const float4* FSI_LAUNCH_RO grid, int p,
-                                         float (*ext)[kTileCap] = nullptr) {
-  __shared__ float own[kExtTile ? 1 : 3][kExtTile ? 1 : kTileCap];
-  float (*tile)[kTileCap] = kExtTile ? ext : reinterpret_cast<float (*)[kTileCap]>(own);
-  __shared__ int sh[8];
+// G2P of particle p from grid velocities: v and the APIC C in the reference's node order, then
+// advection and clamp. row(i, j, in)(k, v): the velocity v of node k of the stencil row (i, j), whose
+// nodes lie in the grid where in[k]. kInside: the whole stencil lies in the grid.
+template <bool kInside, class Row>
+__device__ __forceinline__ void g2p_gather(const Mpm& m, const PView& P, int p, const int base[3],
+                                           const float fx[3], Row row) {
   const long long cap = m.cap;
-  const bool act = p < m.n && P.active[p] != 0;
-  int base[3] = {0, 0, 0};
-  float fx[3] = {0.f, 0.f, 0.f}, x[3] = {0.f, 0.f, 0.f};
-  if (act) {
-    load_particle_x(P, cap, p, x);
-    base_fx(m, x, base, fx);
-  }
-  Box box;
-  if (!cta_box(m, act, base, box, sh)) return;
-  const bool use_tile = box.vol <= kTileCap;
-  if (use_tile) {
-    const int e12 = box.ext[1] * box.ext[2];
-    for (int t = threadIdx.x; t < box.vol; t += blockDim.x) {
-      const int ti = t / e12, r = t - ti * e12, tj = r / box.ext[2], tk = r - tj * box.ext[2];
-      const int i = box.lo[0] + ti, j = box.lo[1] + tj, k = box.lo[2] + tk;
-      float v[3];
-      grid_op(m, grid[node_index(m, i, j, k)], i, j, k, v);
-      tile[0][t] = v[0]; tile[1][t] = v[1]; tile[2][t] = v[2];
-    }
-    __syncthreads();
-  }
-  if (!act) return;
   float nv[3] = {0.f, 0.f, 0.f};
   float nc[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float four_inv_dx = __fmul_rn(4.f, m.inv_dx);
   // Per-axis stencil terms, once per particle; the sums run in the reference's node order.
-  float wa[3][3], dp[3][3];
+  float wa[3][3];
   bool ina[3][3];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int o = 0; o < 3; ++o) {
       wa[a][o] = bspline_w(fx[a], o);
-      dp[a][o] = __fsub_rn((float)o, fx[a]);
       const int n = base[a] + o;
-      ina[a][o] = n >= 0 && n < (a == 0 ? m.nx : (a == 1 ? m.ny : m.nz));
+      ina[a][o] = kInside || (n >= 0 && n < (a == 0 ? m.nx : (a == 1 ? m.ny : m.nz)));
     }
-  const int st1 = use_tile ? box.ext[2] : m.nz;
-  const long long st0 = use_tile ? (long long)box.ext[1] * box.ext[2] : (long long)m.ny * m.nz;
-  const long long t0 = use_tile
-      ? ((long long)(base[0] - box.lo[0]) * box.ext[1] + (base[1] - box.lo[1])) * box.ext[2] + (base[2] - box.lo[2])
-      : ((long long)base[0] * m.ny + base[1]) * m.nz + base[2];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     if (!ina[0][i]) continue;
@@ -818,18 +846,18 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
     for (int j = 0; j < 3; ++j) {
       if (!ina[1][j]) continue;
       const float wxy = __fmul_rn(wa[0][i], wa[1][j]);
+      auto node = row(i, j, ina[2]);
+      // Node offsets made again for each row: nine of them held through the gather spill.
+      float f[3] = {fx[0], fx[1], fx[2]};
+      asm volatile("" : "+f"(f[0]), "+f"(f[1]), "+f"(f[2]));
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         if (!ina[2][k]) continue;
         const float w = __fmul_rn(wxy, wa[2][k]);
-        const long long t = t0 + i * st0 + j * st1 + k;
         float gv[3];
-        if (use_tile) {
-          gv[0] = tile[0][t]; gv[1] = tile[1][t]; gv[2] = tile[2][t];
-        } else {
-          grid_op(m, grid[t], base[0] + i, base[1] + j, base[2] + k, gv);
-        }
-        const float dpos[3] = {dp[0][i], dp[1][j], dp[2][k]};
+        node(k, gv);
+        const float dpos[3] = {__fsub_rn((float)i, f[0]), __fsub_rn((float)j, f[1]),
+                               __fsub_rn((float)k, f[2])};
 #pragma unroll
         for (int a = 0; a < 3; ++a) nv[a] = __fadd_rn(nv[a], __fmul_rn(w, gv[a]));
         const float s = __fmul_rn(four_inv_dx, w);
@@ -845,6 +873,8 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
   for (int a = 0; a < 3; ++a) P.v[a * cap + p] = nv[a];
 #pragma unroll
   for (int i = 0; i < 9; ++i) P.C[i * cap + p] = m.apic ? nc[i] : 0.f;
+  float x[3];  // read again: not held in registers through the gather
+  load_particle_x(P, cap, p, x);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     float xa = __fadd_rn(x[a], __fmul_rn(m.dt, nv[a]));
@@ -853,29 +883,139 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
   }
 }
 
-// Zeroes the dirty ones of the 32 4^3 node blocks from b0 (one warp; its lanes all call it): the
-// flags in one load, then two nodes per lane of each dirty block, and the flags reset.
-__device__ __forceinline__ void clear_dirty_body(const Mpm& m, float4* __restrict__ grid,
-                                                 uint8_t* __restrict__ dirty, long long b0) {
-  const long long nblocks = (long long)m.nbx * m.nby * m.nbz;
-  const int lane = threadIdx.x & 31;
-  const long long mine = b0 + lane;
-  const bool d = mine < nblocks && dirty[mine] != 0;
-  unsigned todo = __ballot_sync(0xffffffffu, d);
-  while (todo) {
-    const int l = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const long long b = b0 + l;
-    const int bi = (int)(b / ((long long)m.nby * m.nbz));
-    const int bj = (int)((b / m.nbz) % m.nby);
-    const int bk = (int)(b % m.nbz);
-#pragma unroll
-    for (int t = lane; t < 64; t += 32) {
-      const int i = bi * 4 + (t >> 4), j = bj * 4 + ((t >> 2) & 3), k = bk * 4 + (t & 3);
-      if (i < m.nx && j < m.ny && k < m.nz) grid[node_index(m, i, j, k)] = make_float4(0.f, 0.f, 0.f, 0.f);
+// Grid update + G2P of particle p (this thread) within its CTA; every thread calls it.
+// Bound by issue: 945 of about 1,500 instructions a warp are the 27 nodes' rounded products and
+// sums, at 71 % of the issue slots; the rest stages the box, with some ten shared-memory wavefronts
+// a node less than a gather straight from the grid (16 a load: the eight particles of a cell read
+// four lines). 2,097,152 particles: 144 us with the tile and the grid behind one test per node,
+// quotients by integer division and boxes held through the gather; 109 as it is. Velocities made
+// by a pass of their own over the dirty blocks gave 105 + 10.
+// A CTA that ends one body and begins the next has a box between the two that does not fit; it
+// stages two boxes instead. Gathering such a CTA straight from the grid, 27 grid updates a particle
+// in a row, took 12 us, longer than the whole launch of a few bodies (now 5).
+// kExtTile: the tile is the caller's shared memory `ext` (3 x kTileCap floats) instead of a
+// static array of its own.
+template <bool kExtTile = false>
+__device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
+                                         const float4* FSI_LAUNCH_RO grid, int p,
+                                         float (*ext)[kTileCap] = nullptr) {
+  __shared__ float own[kExtTile ? 1 : 3][kExtTile ? 1 : kTileCap];
+  float (*tile)[kTileCap] = kExtTile ? ext : reinterpret_cast<float (*)[kTileCap]>(own);
+  __shared__ int sh[16], last[16][4];
+  const bool act = p < m.n && P.active[p] != 0;
+  int base[3] = {0, 0, 0};
+  float fx[3] = {0.f, 0.f, 0.f};
+  if (act) {
+    float x[3];
+    load_particle_x(P, m.cap, p, x);
+    base_fx(m, x, base, fx);
+  }
+  Box box;
+  if (!cta_box(m, act, base, box, sh)) return;
+  bool use_tile = box.vol <= kTileCap;
+  int off = 0;  // this thread's box in the tile
+  // The grid-updated velocities of a box, into the tile from `at`. Quotients of t < kTileCap by
+  // float reciprocals: (t + 1/2) / e is at least 1 / (2 e) from an integer, its rounding error
+  // below 2^-22 t / e.
+  auto stage = [&](const Box& b, int at) {
+    const int e12 = b.ext[1] * b.ext[2];
+    const float r12 = 1.f / (float)e12, r2 = 1.f / (float)b.ext[2];
+    for (int t = threadIdx.x; t < b.vol; t += blockDim.x) {
+      const int ti = (int)(((float)t + 0.5f) * r12), r = t - ti * e12;
+      const int tj = (int)(((float)r + 0.5f) * r2), tk = r - tj * b.ext[2];
+      const int i = b.lo[0] + ti, j = b.lo[1] + tj, k = b.lo[2] + tk;
+      float v[3];
+      grid_op(m, grid[node_index(m, i, j, k)], i, j, k, v);
+      tile[0][at + t] = v[0]; tile[1][at + t] = v[1]; tile[2][at + t] = v[2];
+    }
+  };
+  if (use_tile) {
+    stage(box, 0);
+  } else {
+    Box two[2];
+    const bool part = cut_boxes(m, act, base, two, sh, last);
+    use_tile = two[0].vol + two[1].vol <= kTileCap;
+    if (use_tile) {
+      stage(two[0], 0);
+      stage(two[1], two[0].vol);
+      box = part ? two[1] : two[0];
+      off = part ? two[0].vol : 0;
     }
   }
-  if (d) dirty[mine] = 0;
+  __syncthreads();
+  if (!act) return;
+  if (use_tile) {
+    const int s1 = box.ext[2], s0 = box.ext[1] * s1;
+    const int t0 = off + (base[0] - box.lo[0]) * s0 + (base[1] - box.lo[1]) * s1 + (base[2] - box.lo[2]);
+    auto staged = [&](int i, int j, const bool*) {
+      return [tile, t = t0 + i * s0 + j * s1](int k, float v[3]) {
+        v[0] = tile[0][t + k]; v[1] = tile[1][t + k]; v[2] = tile[2][t + k];
+      };
+    };
+    if (base[0] >= 0 && base[0] + 2 < m.nx && base[1] >= 0 && base[1] + 2 < m.ny && base[2] >= 0 &&
+        base[2] + 2 < m.nz)
+      g2p_gather<true>(m, P, p, base, fx, staged);
+    else
+      g2p_gather<false>(m, P, p, base, fx, staged);
+  } else {
+    // The three nodes of a row are loaded together: one node after another, the 27 latencies of a
+    // single such CTA outlast a small launch.
+    const long long t0 = ((long long)base[0] * m.ny + base[1]) * m.nz + base[2];
+    g2p_gather<false>(m, P, p, base, fx, [&](int i, int j, const bool in[3]) {
+      const long long t = t0 + (long long)i * m.ny * m.nz + (long long)j * m.nz;
+      struct { float4 n[3]; } r;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) r.n[k] = in[k] ? grid[t + k] : make_float4(0.f, 0.f, 0.f, 0.f);
+      return [&m, &base, r, i, j](int k, float v[3]) {
+        grid_op(m, r.n[k], base[0] + i, base[1] + j, base[2] + k, v);
+      };
+    });
+  }
+}
+
+// The dirty ones of the 4^3 node blocks [b0, b0 + kBlock) (each of the CTA's kBlock threads looks
+// at one), listed in shared memory by their first node, so that the whole CTA works on them:
+// a body's blocks lie together.
+struct DirtyList {
+  int n;
+  int3 first[kBlock];
+};
+
+__device__ __forceinline__ void list_dirty(const Mpm& m, const uint8_t* dirty, long long b, DirtyList& l) {
+  __syncthreads();  // a previous list is no longer read
+  if (threadIdx.x == 0) l.n = 0;
+  __syncthreads();
+  const bool d = b < (long long)m.nbx * m.nby * m.nbz && dirty[b] != 0;
+  const unsigned mask = __ballot_sync(0xffffffffu, d);
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0 && mask) at = atomicAdd(&l.n, __popc(mask));
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(mask & ((1u << lane) - 1u));
+  if (d) {
+    const int bi = (int)(b / ((long long)m.nby * m.nbz)), r = (int)(b - (long long)bi * m.nby * m.nbz);
+    const int bj = r / m.nbz, bk = r - bj * m.nbz;
+    l.first[at] = make_int3(4 * bi, 4 * bj, 4 * bk);
+  }
+  __syncthreads();
+}
+
+// Node e of the list: its coordinates, and whether it lies in the grid.
+__device__ __forceinline__ bool list_node(const Mpm& m, const DirtyList& l, int e, int& i, int& j, int& k) {
+  if (e >= 64 * l.n) return false;
+  const int3 f = l.first[e >> 6];
+  i = f.x + ((e >> 4) & 3); j = f.y + ((e >> 2) & 3); k = f.z + (e & 3);
+  return i < m.nx && j < m.ny && k < m.nz;
+}
+
+// Zeroes the dirty blocks and their flags.
+__device__ __forceinline__ void clear_dirty_body(const Mpm& m, float4* __restrict__ grid,
+                                                 uint8_t* __restrict__ dirty, long long b, DirtyList& l) {
+  list_dirty(m, dirty, b, l);
+  for (int e = threadIdx.x; e < 64 * l.n; e += kBlock) {
+    int i, j, k;
+    if (list_node(m, l, e, i, j, k)) grid[node_index(m, i, j, k)] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (b < (long long)m.nbx * m.nby * m.nbz && dirty[b] != 0) dirty[b] = 0;
 }
 
 // Host-side validation of a solver descriptor and its particle arrays.
