@@ -361,8 +361,9 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
 // Each CTA (one per SM) takes a contiguous range of (column, x) plane steps. Warps 0-15 run
 // the epilogues (warp w reads TMEM lanes 32 (w % 4) .. + 31 and columns 16 (w / 4) .. + 15);
 // one thread of warp 16 issues the plane copies and layers 2-4 of each tile as its layer-1,
-// -2 and -3 epilogues finish; one thread of warp 17 issues layer 1 (42 MMAs) of the tiles
-// ahead, as soon as the tensor-memory half and the planes a tile needs are free and loaded.
+// -2 and -3 epilogues finish; one thread each of warps 17 and 18 issues layer 1 (42 MMAs) of the
+// even and odd tiles, as soon as the tensor-memory half and the planes a tile needs are free and
+// loaded.
 // Two tiles are in flight (TMEM halves 0 and 256): the tensor cores run layer 1 of tile
 // t + 1 while the epilogues of tile t run on the CUDA cores, and the small layers of tile t
 // never queue behind a thread that is blocked issuing layer 1. Every hand-over is an
@@ -386,7 +387,7 @@ constexpr int kWorkers = 32 * kEpiWarps;
 constexpr int kGroupWarps = kEpiWarps / 2;            // two epilogue groups, alternate tiles
 constexpr size_t kHBytes = 128 * 64 * 2;              // one activation tile
 constexpr int kChainWarp = kEpiWarps, kL1Warp = kEpiWarps + 1;
-constexpr int kInferThreads = kWorkers + 64;          // + the two MMA-issuing warps
+constexpr int kInferThreads = kWorkers + 96;          // + the three MMA-issuing warps
 constexpr uint32_t kPlaneBytes = 3u * kPlaneRows * 16u;  // one plane: three tensor-copy boxes
 static_assert(kL1Chunk * 3 == kL1Mmas, "layer 1 is issued in three equal chunks");
 // Highest row read: the last tile's last row, offset +35, and the +16-byte second half of
@@ -655,10 +656,11 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 }
 
 // Chain-issuer state of one epilogue group: its next tile, the epilogue of that tile it
-// waits for (0-2), phases of its hand-over barrier waited and commits to its layer barrier.
+// waits for (0-2), phases of its hand-over barrier waited, commits to its layer barrier, and
+// the last tile whose layer 1 is known to be complete.
 struct Group {
   uint32_t tile, stage = 0, n_h = 0, c_l = 0;
-  Segment seg;
+  int l1_done = -1;
 };
 
 struct ChainCtx {
@@ -684,46 +686,63 @@ __device__ __forceinline__ void fill_segment_start(const CUtensorMap* map, uint3
   }
 }
 
-// If group H has handed over its next epilogue, issues the layer that follows it (and, after
-// a layer-1 epilogue, the plane copies that tile frees); returns whether it did.
+// Plane copies still to come: the segment they belong to and the next plane step q >= 1 whose
+// plane xs + q + 2 replaces plane xs + q - 2.
+struct FillCursor {
+  Segment seg;
+  int q = 1;
+};
+
+// Issues the plane copies whose slots are free. Plane xs + q + 2 takes the slot of the oldest
+// plane of step q - 1, so the tiles of every step before q must have read their planes; the first
+// planes of the next segment take all slots after the segment's last tile. Layer 1 of even and
+// odd tiles is issued by two threads, so completion is tracked for both.
+__device__ __forceinline__ void advance_fills(FillCursor& f, const Group& even, const Group& odd,
+                                              const ChainCtx& cx, uint32_t& fills, const LbmGeom& g,
+                                              const RowGeom& rg) {
+  auto complete = [&](int last) {  // layer 1 of every tile up to `last`
+    const int e = last & ~1, o = (last & 1) ? last : last - 1;
+    return even.l1_done >= e && (o < 0 || odd.l1_done >= o);
+  };
+  while (true) {
+    const Segment& s = f.seg;
+    if (f.q + 1 < s.nq) {
+      if (!complete((int)s.first + kPlaneTiles * f.q - 1)) return;
+      const int sl = (f.q + 3) & 3;
+      fill_plane(cx.map, cx.s_rows, &cx.bar_rows[sl], sl, wrap(s.xs + f.q + 2, g.nx), s.y0, s.z0);
+      fills ^= 1u << sl;
+      ++f.q;
+    } else {
+      if (s.p0 + s.nq >= cx.w1 || !complete((int)(s.first + s.ntile) - 1)) return;
+      f.seg = segment_at(s.p0 + s.nq, cx.w1, s.first + s.ntile, g, rg);
+      f.q = 1;
+      fill_segment_start(cx.map, cx.s_rows, cx.bar_rows, fills, f.seg, g.nx);
+    }
+  }
+}
+
+// If group H has handed over its next epilogue, issues the layer that follows it; returns whether
+// it did.
 template <int H>
-__device__ __forceinline__ bool serve(Group& gr, uint64_t& bar_h, uint64_t& bar_l, uint64_t dh, const ChainCtx& cx,
-                                      uint32_t& fills, const LbmGeom& g, const RowGeom& rg) {
+__device__ __forceinline__ bool serve(Group& gr, uint64_t& bar_h, uint64_t& bar_l, uint64_t dh, const ChainCtx& cx) {
   if (gr.tile >= cx.ntiles || !mbar_test(&bar_h, gr.n_h & 1)) return false;
   ++gr.n_h;
   tc::fence_after_sync();
   const uint32_t tb = cx.tmem + ((uint32_t)H << 8);
-  if (gr.stage == 0) {  // layer-1 epilogue done: layer 2, plane copies
+  if (gr.stage == 0) {  // layer-1 epilogue done
     issue_layer(tb + 64, dh, cx.w2, kIdesc64);
-    tc::mma_commit(&bar_l);
-    ++gr.c_l;
-    seek(gr.seg, gr.tile, cx.w1, g, rg);
-    const Segment& s = gr.seg;
-    const int ti = (int)(gr.tile - s.first), q = ti / kPlaneTiles, m = ti - q * kPlaneTiles;
-    // Layer 1 of this tile is complete, so is every earlier one: plane step q - 1's oldest
-    // plane gives its slot to plane xs + q + 2; after a segment's last tile, the next
-    // segment's first planes go in.
-    if (m == 0 && q >= 1 && q + 1 < s.nq) {
-      const int sl = (q + 3) & 3;
-      fill_plane(cx.map, cx.s_rows, &cx.bar_rows[sl], sl, wrap(s.xs + q + 2, g.nx), s.y0, s.z0);
-      fills ^= 1u << sl;
-    }
-    if ((uint32_t)ti + 1 == s.ntile && s.p0 + s.nq < cx.w1)
-      fill_segment_start(cx.map, cx.s_rows, cx.bar_rows, fills, segment_at(s.p0 + s.nq, cx.w1, s.first + s.ntile, g, rg),
-                         g.nx);
+    gr.l1_done = (int)gr.tile;
     gr.stage = 1;
   } else if (gr.stage == 1) {
     issue_layer(tb + 128, dh, cx.w3, kIdesc64);
-    tc::mma_commit(&bar_l);
-    ++gr.c_l;
     gr.stage = 2;
   } else {
     issue_layer(tb + 192, dh, cx.w4, kIdesc32);
-    tc::mma_commit(&bar_l);
-    ++gr.c_l;
     gr.stage = 0;
     gr.tile += 2;
   }
+  tc::mma_commit(&bar_l);
+  ++gr.c_l;
   return true;
 }
 
@@ -795,22 +814,22 @@ __global__ void __launch_bounds__(kInferThreads, 1) closure_infer_kernel(InferAr
       uint32_t fills = 0;  // parity of the copies issued per slot
       bool ok = true;
       Group gr0, gr1;
+      FillCursor fc;
       gr0.tile = 0;
       gr1.tile = 1;
       if (ntiles > 0) {
         // The first segment's planes: ordinal u is plane xs - 1 + u, in slot u & 3.
-        const Segment s0 = segment_at(w0, w1, 0, g, rg);
-        fill_segment_start(&rows_map, sRows, bar_rows, fills, s0, g.nx);
-        gr0.seg = s0;
-        gr1.seg = s0;
+        fc.seg = segment_at(w0, w1, 0, g, rg);
+        fill_segment_start(&rows_map, sRows, bar_rows, fills, fc.seg, g.nx);
       }
       const ChainCtx cx{&rows_map, sRows, bar_rows, tmem, dW2, dW3, dW4, w1, ntiles};
       long long t_idle = clock64();
       // Serve the two epilogue groups in the order their hand-overs arrive.
       while (gr0.tile < ntiles || gr1.tile < ntiles) {
-        const bool p0 = serve<0>(gr0, bar_h[0], bar_l[0], dH0, cx, fills, g, rg);
-        const bool p1 = serve<1>(gr1, bar_h[1], bar_l[1], dH1, cx, fills, g, rg);
+        const bool p0 = serve<0>(gr0, bar_h[0], bar_l[0], dH0, cx);
+        const bool p1 = serve<1>(gr1, bar_h[1], bar_l[1], dH1, cx);
         if (p0 || p1) {
+          advance_fills(fc, gr0, gr1, cx, fills, g, rg);
           t_idle = clock64();
         } else if (*abort) {
           ok = false;
@@ -831,46 +850,50 @@ __global__ void __launch_bounds__(kInferThreads, 1) closure_infer_kernel(InferAr
         if (gr1.c_l > 0) tc::mbar_wait(&bar_l[1], (gr1.c_l - 1) & 1, nullptr, 0);
       }
     }
-  } else if (warp == kL1Warp) {
+  } else if (warp >= kL1Warp) {
     // ------------------------------------------------------------------ layer 1
+    // Tiles of parity h, into TMEM half h. One thread issues an MMA in about 86 cycles, while
+    // its operands (6 KB at 128 bytes a cycle from shared memory) take 48: with a thread for either
+    // parity the inference of 192x96x96 cells takes 283 us, against 297 with one thread for both.
+    const int h = warp - kL1Warp;
     if (lane == 0) {
       const uint64_t dRows = tc::smem_desc(sRows, 0u, 128u);
       const uint64_t dW1 = tc::smem_desc(tc::smem_addr(smem + kOffW1), 128u, 256u);
-      uint32_t tile = 0, rows_phase = 0, issued = 0;
+      uint32_t first = 0, rows_phase = 0, issued = 0;
       bool ok = true;
 #define FSI_WAIT_ROWS(sl) (ok = tc::mbar_wait_abortable(&bar_rows[(sl)], (rows_phase >> (sl)) & 1u, abort, a.err, 12), rows_phase ^= 1u << (sl), ok)
       for (int p0 = w0; p0 < w1 && ok;) {
         const int nq = min(g.nx - p0 % g.nx, w1 - p0);
-        const int ntile = kPlaneTiles * nq;
-        for (int ti = 0; ti < ntile; ++ti, ++tile) {
-          const int q = ti / kPlaneTiles, m = ti - q * kPlaneTiles;
-          const uint32_t h = tile & 1;
-          // The TMEM half's previous tile (tile - 2) has been read by its layer-1 epilogue.
-          if (tile >= 2 && !(ok = tc::mbar_wait_abortable(&bar_e1[h], ((tile - 2) >> 1) & 1u, abort, a.err, 14))) break;
-          // The planes of this plane step are loaded.
-          if (ti == 0) {
+        for (int q = 0; q < nq && ok; ++q) {
+          // The planes of this plane step are loaded (each step has a tile of either parity, so
+          // both threads see every phase).
+          if (q == 0) {
             if (!FSI_WAIT_ROWS(0) || !FSI_WAIT_ROWS(1) || !FSI_WAIT_ROWS(2)) break;
-          } else if (m == 0 && !FSI_WAIT_ROWS((q + 2) & 3)) {
+          } else if (!FSI_WAIT_ROWS((q + 2) & 3)) {
             break;
           }
-          tc::fence_after_sync();
-          const int base = kPadLo + kLine + 128 * m;
-          const int r0 = base + (q & 3) * kSlotRows, r1 = base + ((q + 1) & 3) * kSlotRows,
-                    r2 = base + ((q + 2) & 3) * kSlotRows;
-          const uint32_t d = tmem + (h << 8);
-          issue_l1_chunk<0>(d, dRows, r0, r1, r2, dW1);
-          issue_l1_chunk<1>(d, dRows, r0, r1, r2, dW1);
-          issue_l1_chunk<2>(d, dRows, r0, r1, r2, dW1);
-          tc::mma_commit(&bar_l1[h]);
-          ++issued;
+          for (int m = 0; m < kPlaneTiles; ++m) {
+            const uint32_t tile = first + (uint32_t)(kPlaneTiles * q + m);
+            if ((int)(tile & 1) != h) continue;
+            // The TMEM half's previous tile (tile - 2) has been read by its layer-1 epilogue.
+            if (tile >= 2 && !(ok = tc::mbar_wait_abortable(&bar_e1[h], ((tile - 2) >> 1) & 1u, abort, a.err, 14))) break;
+            tc::fence_after_sync();
+            const int base = kPadLo + kLine + 128 * m;
+            const int r0 = base + (q & 3) * kSlotRows, r1 = base + ((q + 1) & 3) * kSlotRows,
+                      r2 = base + ((q + 2) & 3) * kSlotRows;
+            const uint32_t d = tmem + ((uint32_t)h << 8);
+            issue_l1_chunk<0>(d, dRows, r0, r1, r2, dW1);
+            issue_l1_chunk<1>(d, dRows, r0, r1, r2, dW1);
+            issue_l1_chunk<2>(d, dRows, r0, r1, r2, dW1);
+            tc::mma_commit(&bar_l1[h]);
+            ++issued;
+          }
         }
+        first += (uint32_t)(kPlaneTiles * nq);
         p0 += nq;
       }
-      if (!ok && issued > 0) {
-        // Let the last layer 1 issued (tile issued - 1; tiles go in order) finish (bounded).
-        const uint32_t lt = issued - 1;
-        tc::mbar_wait(&bar_l1[lt & 1], (lt >> 1) & 1u, nullptr, 0);
-      }
+      // Let the last layer 1 issued (this thread's tiles go in order) finish (bounded).
+      if (!ok && issued > 0) tc::mbar_wait(&bar_l1[h], (issued - 1) & 1u, nullptr, 0);
 #undef FSI_WAIT_ROWS
     }
   } else {
