@@ -217,16 +217,18 @@ __global__ void __launch_bounds__(kBlock)
                    t.first + (int)threadIdx.x, l);
 }
 
-// Three blocks per SM: 187 us for 64 scenes, against 212 at its natural 101 registers (two) and 210
-// at 64 (four, spills).
-__global__ void __launch_bounds__(kBlock, 3)
+// Four blocks per SM: 157 us for 64 scenes, against 160 with three and 158 with five (187 with the
+// lattice read directly).
+__global__ void __launch_bounds__(kBlock, 4)
     batch_coupling_forces_kernel(const BatchLattice* __restrict__ lat,
                                  const BatchSolid* __restrict__ sol, const Tile* __restrict__ ptiles,
                                  ForceArgs base, float dt_ratio, int build_fraction) {
   const Tile t = ptiles[blockIdx.x];
   const ForceArgs a = scene_force_args(base, lat[t.lattice], sol[t.lattice], t.lattice, dt_ratio,
                                        build_fraction);
-  coupling_forces_body<false>(a, t.first * kBlock + threadIdx.x);
+  __shared__ float tile[3][kTileCap];
+  __shared__ StageScratch scratch;
+  coupling_staged_body(a, t.first * kBlock + threadIdx.x, tile, scratch);
 }
 
 __global__ void __launch_bounds__(kTileCells)

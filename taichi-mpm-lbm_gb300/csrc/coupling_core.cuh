@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 #include "fsi_common.cuh"
 
 namespace fsi {
@@ -68,6 +69,28 @@ __host__ __device__ constexpr int stencil_flag_bit(int s) {
   return -1;
 }
 
+// The bits of stencil_flag_bit: none set in a flag word, all 27 nodes are fluid.
+__host__ __device__ constexpr uint32_t stencil_flag_mask() {
+  uint32_t m = 0;
+  for (int s = 0; s < 27; ++s) m |= 1u << stencil_flag_bit(s);
+  return m;
+}
+constexpr uint32_t kAllUsable = (1u << 27) - 1u;
+
+// Where coupling_particle takes its inputs from: memory, as they are needed. ok: the stencil's
+// lattice velocities are at hand (operator()); kBatch: else this many of their loads go out
+// together.
+struct FromMemory {
+  static constexpr bool ok = false;
+  static constexpr int kBatch = 9;
+  __device__ __forceinline__ void operator()(int, int, int, float*) const {}
+  __device__ __forceinline__ float x(const ForceArgs& a, int p, int ax) const { return a.x[ax * a.cap + p]; }
+  __device__ __forceinline__ float v(const ForceArgs& a, int p, int ax) const { return a.v[ax * a.cap + p]; }
+  __device__ __forceinline__ float mass(const ForceArgs& a, int p) const { return a.mass[p]; }
+  __device__ __forceinline__ float vol(const ForceArgs& a, int p) const { return a.vol[p]; }
+  __device__ __forceinline__ uint32_t flag(const ForceArgs& a, long long c) const { return a.flags[c]; }
+};
+
 // The per-particle part of _compute_coupling_forces_kernel (fsi/coupling.py:336-387) for
 // active particle p: interpolates the fluid velocity over the in-grid fluid nodes of its
 // stencil, and if the valid weight exceeds min_valid_weight computes the penalty force with
@@ -79,13 +102,13 @@ __host__ __device__ constexpr int stencil_flag_bit(int s) {
 // up front (fewer dependent round trips, more registers: for launches with few particles,
 // where latency and not occupancy bounds the kernel). Every path sums the same values in the
 // same order.
-template <bool kGatherAhead>
+template <bool kGatherAhead, class In = FromMemory>
 __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int base[3],
                                                   float wv[3][3], uint32_t& usable, float& valid,
                                                   float pf[3], bool& partial, bool& clipped,
-                                                  bool& unsupported) {
+                                                  bool& unsupported, const In& in = {}) {
   const long long cap = a.cap;
-  const float x[3] = {a.x[p], a.x[cap + p], a.x[2 * cap + p]};
+  const float x[3] = {in.x(a, p, 0), in.x(a, p, 1), in.x(a, p, 2)};
   float fx[3];
   stencil_base(a.c.inv_dx, x, base, fx);
 #pragma unroll
@@ -103,30 +126,44 @@ __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int
     // nodes at a time) after one dependent load; the sums run in stencil order.
     const long long sx = (long long)a.g.ny * a.g.nz, sy = a.g.nz;
     const long long c1 = (base[0] + 1) * sx + (base[1] + 1) * sy + (base[2] + 1);
-    const uint32_t fl = a.flags[c1];
+    const uint32_t fl = in.flag(a, c1);
+    const float4* FSI_LAUNCH_RO m0 = a.macro + (c1 - sx - sy - 1);
+    // kFull: every node counts, with no test per node (all but the particles beside a wall).
+    auto gather = [&](auto kFull, auto kB, auto velocity) {
+#pragma unroll
+      for (int b = 0; b < 27 / kB(); ++b) {
+        float u[kB()][3];
+#pragma unroll
+        for (int t = 0; t < kB(); ++t) {
+          const int s = kB() * b + t;
+          if (kFull() || ((usable >> s) & 1u)) velocity(s / 9, (s / 3) % 3, s % 3, u[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < kB(); ++t) {
+          const int s = kB() * b + t, i = s / 9, j = (s / 3) % 3, k = s % 3;
+          if (!kFull() && !((usable >> s) & 1u)) continue;
+          const float w = __fmul_rn(__fmul_rn(wv[0][i], wv[1][j]), wv[2][k]);
+          valid = __fadd_rn(valid, w);
+#pragma unroll
+          for (int ax = 0; ax < 3; ++ax) uf[ax] = __fadd_rn(uf[ax], __fmul_rn(w, u[t][ax]));
+        }
+      }
+    };
+    auto memory = [&](int i, int j, int k, float v[3]) {
+      const float4 mc = m0[i * sx + j * sy + k];
+      v[0] = mc.x; v[1] = mc.y; v[2] = mc.z;
+    };
+    using Ahead = std::integral_constant<int, In::kBatch>;  // loads of memory that go out together
+    using One = std::integral_constant<int, 1>;
+    const bool full = (fl & stencil_flag_mask()) == 0;
 #pragma unroll
     for (int s = 0; s < 27; ++s) usable |= ((~fl >> stencil_flag_bit(s)) & 1u) << s;
-    constexpr int kB = 9;
-    const float4* FSI_LAUNCH_RO m0 = a.macro + (c1 - sx - sy - 1);
-#pragma unroll
-    for (int b = 0; b < 27 / kB; ++b) {
-      float4 mc[kB];
-#pragma unroll
-      for (int t = 0; t < kB; ++t) {
-        const int s = kB * b + t, i = s / 9, j = (s / 3) % 3, k = s % 3;
-        if ((usable >> s) & 1u) mc[t] = m0[i * sx + j * sy + k];
-      }
-#pragma unroll
-      for (int t = 0; t < kB; ++t) {
-        const int s = kB * b + t, i = s / 9, j = (s / 3) % 3, k = s % 3;
-        if (!((usable >> s) & 1u)) continue;
-        const float w = __fmul_rn(__fmul_rn(wv[0][i], wv[1][j]), wv[2][k]);
-        valid = __fadd_rn(valid, w);
-        uf[0] = __fadd_rn(uf[0], __fmul_rn(w, mc[t].x));
-        uf[1] = __fadd_rn(uf[1], __fmul_rn(w, mc[t].y));
-        uf[2] = __fadd_rn(uf[2], __fmul_rn(w, mc[t].z));
-      }
-    }
+    if (!in.ok)
+      gather(std::false_type{}, Ahead{}, memory);
+    else if (full)
+      gather(std::true_type{}, One{}, in);
+    else
+      gather(std::false_type{}, One{}, in);
   } else if (!kGatherAhead) {
 #pragma unroll
     for (int s = 0; s < 27; ++s) {
@@ -153,9 +190,9 @@ __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int
     for (int s = 0; s < 27; ++s) {
       const int i = s / 9, j = (s / 3) % 3, k = s % 3;
       const int ni = base[0] + i, nj = base[1] + j, nk = base[2] + k;
-      const bool in = ni >= 0 && ni < a.g.nx && nj >= 0 && nj < a.g.ny && nk >= 0 && nk < a.g.nz;
-      inside |= (uint32_t)in << s;
-      fl[s] = in ? a.flags[((long long)ni * a.g.ny + nj) * a.g.nz + nk] : kFlagSolid;
+      const bool here = ni >= 0 && ni < a.g.nx && nj >= 0 && nj < a.g.ny && nk >= 0 && nk < a.g.nz;
+      inside |= (uint32_t)here << s;
+      fl[s] = here ? a.flags[((long long)ni * a.g.ny + nj) * a.g.nz + nk] : kFlagSolid;
     }
 #pragma unroll
     for (int s = 0; s < 27; ++s)
@@ -193,7 +230,7 @@ __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
     uf[ax] = __fdiv_rn(uf[ax], valid);
-    dv[ax] = __fsub_rn(uf[ax], a.v[ax * cap + p]);
+    dv[ax] = __fsub_rn(uf[ax], in.v(a, p, ax));
   }
   if (a.c.use_rel_limit) {
     const float nrm = norm3(dv[0], dv[1], dv[2]);
@@ -203,7 +240,7 @@ __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int
       clipped = true;
     }
   }
-  const float gm = __fmul_rn(a.c.gamma_eff, a.mass[p]);
+  const float gm = __fmul_rn(a.c.gamma_eff, in.mass(a, p));
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) pf[ax] = __fmul_rn(gm, dv[ax]);
   if (a.c.use_force_limit) {
@@ -222,10 +259,12 @@ __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int
 
 // Reaction force xyz and solid-fraction term (w) that a coupled particle with stencil weight
 // w, valid weight `valid` and force pf spreads into one fluid node (coupling.py:389-400).
+// kUnitCell: the caller knows that the cell volume is 1.
+template <bool kUnitCell = false>
 __device__ __forceinline__ float4 coupling_spread_terms(const fsi_coupling_desc& c, float w,
                                                         float valid, const float pf[3], float vp) {
   // x / 1 is exactly x: the divisions by the cell volume are skipped for unit cells (dx = 1).
-  const bool unit_cell = c.cell_volume == 1.0f;
+  const bool unit_cell = kUnitCell || c.cell_volume == 1.0f;
   const float nw = __fdiv_rn(w, valid);
   float add[3];
 #pragma unroll
@@ -241,8 +280,8 @@ __device__ __forceinline__ float4 coupling_spread_terms(const fsi_coupling_desc&
 // _compute_coupling_forces_kernel, fsi/coupling.py:332-406, for particle p (this thread);
 // every lane of the warp calls it (warp-aggregated counters). The reaction and solid
 // fraction are spread with vector atomics (order of arrival).
-template <bool kGatherAhead>
-__device__ __forceinline__ void coupling_forces_body(const ForceArgs& a, int p) {
+template <bool kGatherAhead, class In = FromMemory>
+__device__ __forceinline__ void coupling_forces_body(const ForceArgs& a, int p, const In& in = {}) {
   const bool live = p < a.n;
   const long long cap = a.cap;
   bool partial = false, clipped = false, unsupported = false;
@@ -254,19 +293,25 @@ __device__ __forceinline__ void coupling_forces_body(const ForceArgs& a, int p) 
       float wv[3][3], valid, pf[3];
       uint32_t usable;
       if (coupling_particle<kGatherAhead>(a, p, base, wv, usable, valid, pf, partial, clipped,
-                                          unsupported)) {
-        const float vp = a.vol[p];
+                                          unsupported, in)) {
+        const float vp = in.vol(a, p);
+        auto spread = [&](auto kFull) {
 #pragma unroll
-        for (int s = 0; s < 27; ++s) {
-          if (!(usable & (1u << s))) continue;
-          const int i = s / 9, j = (s / 3) % 3, k = s % 3;
-          const long long c =
-              ((long long)(base[0] + i) * a.g.ny + (base[1] + j)) * a.g.nz + (base[2] + k);
-          const float w = __fmul_rn(__fmul_rn(wv[0][i], wv[1][j]), wv[2][k]);
-          float4 t = coupling_spread_terms(a.c, w, valid, pf, vp);
-          if (!a.c.build_fraction) t.w = 0.f;
-          red_add_v4(a.accum + c, t.x, t.y, t.z, t.w);
-        }
+          for (int s = 0; s < 27; ++s) {
+            if (!kFull() && !(usable & (1u << s))) continue;
+            const int i = s / 9, j = (s / 3) % 3, k = s % 3;
+            const long long c =
+                ((long long)(base[0] + i) * a.g.ny + (base[1] + j)) * a.g.nz + (base[2] + k);
+            const float w = __fmul_rn(__fmul_rn(wv[0][i], wv[1][j]), wv[2][k]);
+            float4 t = coupling_spread_terms<kFull()>(a.c, w, valid, pf, vp);
+            if (!a.c.build_fraction) t.w = 0.f;
+            red_add_v4(a.accum + c, t.x, t.y, t.z, t.w);
+          }
+        };
+        if (usable == kAllUsable && a.c.cell_volume == 1.0f)
+          spread(std::true_type{});
+        else
+          spread(std::false_type{});
       }
     }
   }

@@ -41,9 +41,12 @@ __global__ void __launch_bounds__(kT, 1024 / kT) p2g_kernel(Mpm m, PView P,
                     *reinterpret_cast<ScatterSmem<kT>*>(scatter_smem));
 }
 
-// The penalty coupling alone (one thread per particle), before p2g_kernel on large launches.
-__global__ void __launch_bounds__(kBlock) coupling_only_kernel(ForceArgs fa) {
-  coupling_forces_body<false>(fa, blockIdx.x * kBlock + threadIdx.x);
+// The penalty coupling alone (one thread per particle), before p2g_kernel on large launches. Four
+// blocks per SM: 79 us for 502,304 particles, against 84 with three and 78 with five (spills).
+__global__ void __launch_bounds__(kBlock, 4) coupling_only_kernel(ForceArgs fa) {
+  __shared__ float tile[3][kTileCap];
+  __shared__ StageScratch scratch;
+  coupling_staged_body(fa, blockIdx.x * kBlock + threadIdx.x, tile, scratch);
 }
 
 // The coupling split in two lighter kernels: the force (gathers), then the spread (vector

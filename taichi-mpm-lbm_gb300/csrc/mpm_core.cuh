@@ -195,7 +195,8 @@ struct Box {
 };
 
 // The part in the grid of the box [sh[0..2], sh[3..5]]; vol: its nodes, at most kTileCap + 1.
-__device__ __forceinline__ Box box_of(const Mpm& m, const int* sh) {
+template <class G>
+__device__ __forceinline__ Box box_of(const G& m, const int* sh) {
   Box box;
   const int n[3] = {m.nx, m.ny, m.nz};
   long long vol = 1;
@@ -210,7 +211,8 @@ __device__ __forceinline__ Box box_of(const Mpm& m, const int* sh) {
   return box;
 }
 
-__device__ bool cta_box(const Mpm& m, bool act, const int base[3], Box& box, int* sh) {
+template <class G>
+__device__ bool cta_box(const G& m, bool act, const int base[3], Box& box, int* sh) {
   // sh: 6 ints of shared scratch
   if (threadIdx.x < 3) { sh[threadIdx.x] = 0x7fffffff; sh[3 + threadIdx.x] = -0x7fffffff; }
   __syncthreads();
@@ -232,7 +234,8 @@ __device__ bool cta_box(const Mpm& m, bool act, const int base[3], Box& box, int
 // begin the next: cuts it in two where consecutive particles are farthest apart. Returns this
 // thread's part (false: before the cut) and both boxes; every thread calls it.
 // sh: 13 ints of shared scratch, last: 4 ints per warp.
-__device__ bool cut_boxes(const Mpm& m, bool act, const int base[3], Box box[2], int* sh, int (*last)[4]) {
+template <class G>
+__device__ bool cut_boxes(const G& m, bool act, const int base[3], Box box[2], int* sh, int (*last)[4]) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   __syncthreads();  // the whole box's scratch is no longer read
   if (t < 12) sh[t] = t % 6 < 3 ? 0x7fffffff : -0x7fffffff;
@@ -279,6 +282,69 @@ __device__ bool cut_boxes(const Mpm& m, bool act, const int base[3], Box box[2],
     if (sh[6 * h] == 0x7fffffff) box[h].vol = 0;
   }
   return part;
+}
+
+// Shared scratch of stage_stencils.
+struct StageScratch {
+  int box[16], last[16][4];
+};
+
+// The 3-vectors of a CTA's stencil nodes in shared memory: node (i, j, k) of this thread's stencil
+// is at t0 + i s0 + j s1 + k. ok: the stencils fit the tile.
+struct Staged {
+  const float (*tile)[kTileCap];
+  bool any, ok;  // any: the CTA has an active particle
+  int t0, s0, s1;
+  __device__ __forceinline__ void operator()(int i, int j, int k, float v[3]) const {
+    const int t = t0 + i * s0 + j * s1 + k;
+    v[0] = tile[0][t]; v[1] = tile[1][t]; v[2] = tile[2][t];
+  }
+};
+
+// Stages the box of the CTA's stencils (two boxes where it ends one body and begins the next), every
+// node once: load(i, j, k, v). Every thread calls it.
+template <class G, class Load>
+__device__ __forceinline__ Staged stage_stencils(const G& m, bool act, const int base[3],
+                                                 float (*tile)[kTileCap], StageScratch& sc, Load load) {
+  Staged st;
+  st.tile = tile;
+  st.ok = false;
+  Box box;
+  st.any = cta_box(m, act, base, box, sc.box);
+  if (!st.any) return st;
+  // A box's nodes into the tile from `at`. Quotients of t < kTileCap by float reciprocals: (t + 1/2) / e
+  // is at least 1 / (2 e) from an integer, its rounding error below 2^-22 t / e.
+  auto stage = [&](const Box& b, int at) {
+    const int e12 = b.ext[1] * b.ext[2];
+    const float r12 = 1.f / (float)e12, r2 = 1.f / (float)b.ext[2];
+    for (int t = threadIdx.x; t < b.vol; t += blockDim.x) {
+      const int ti = (int)(((float)t + 0.5f) * r12), r = t - ti * e12;
+      const int tj = (int)(((float)r + 0.5f) * r2), tk = r - tj * b.ext[2];
+      float v[3];
+      load(b.lo[0] + ti, b.lo[1] + tj, b.lo[2] + tk, v);
+      tile[0][at + t] = v[0]; tile[1][at + t] = v[1]; tile[2][at + t] = v[2];
+    }
+  };
+  st.ok = box.vol <= kTileCap;
+  int off = 0;  // this thread's box in the tile
+  if (st.ok) {
+    stage(box, 0);
+  } else {
+    Box two[2];
+    const bool part = cut_boxes(m, act, base, two, sc.box, sc.last);
+    st.ok = two[0].vol + two[1].vol <= kTileCap;
+    if (st.ok) {
+      stage(two[0], 0);
+      stage(two[1], two[0].vol);
+      box = part ? two[1] : two[0];
+      off = part ? two[0].vol : 0;
+    }
+  }
+  __syncthreads();
+  st.s1 = box.ext[2];
+  st.s0 = box.ext[1] * box.ext[2];
+  st.t0 = off + (base[0] - box.lo[0]) * st.s0 + (base[1] - box.lo[1]) * st.s1 + (base[2] - box.lo[2]);
+  return st;
 }
 
 __device__ __forceinline__ void load_particle_x(const PView& P, long long cap, int p, float x[3]) {
@@ -573,13 +639,14 @@ __device__ __forceinline__ void p2g_runs_body(const Mpm& m, const PView& P, floa
                                               uint8_t* __restrict__ dirty, int p,
                                               ScatterSmem<kT>& sm) {
   const long long cap = m.cap;
-  const bool act = p < m.n && P.active[p] != 0;
+  bool act = false;
   int base[3] = {0, 0, 0};
   float fx[3] = {0.f, 0.f, 0.f};
-  if (act) {
-    float x[3];
+  if (p < m.n) {
+    float x[3];  // beside the flag, not after it
     load_particle_x(P, cap, p, x);
-    base_fx(m, x, base, fx);
+    act = P.active[p] != 0;
+    if (act) base_fx(m, x, base, fx);
   }
   const bool in = act && stencil_in_grid(m.nx, m.ny, m.nz, base);
   const CellOrder o = cell_order(in, base, sm);
@@ -901,57 +968,22 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
                                          float (*ext)[kTileCap] = nullptr) {
   __shared__ float own[kExtTile ? 1 : 3][kExtTile ? 1 : kTileCap];
   float (*tile)[kTileCap] = kExtTile ? ext : reinterpret_cast<float (*)[kTileCap]>(own);
-  __shared__ int sh[16], last[16][4];
-  const bool act = p < m.n && P.active[p] != 0;
+  __shared__ StageScratch scratch;
+  bool act = false;
   int base[3] = {0, 0, 0};
   float fx[3] = {0.f, 0.f, 0.f};
-  if (act) {
-    float x[3];
+  if (p < m.n) {
+    float x[3];  // beside the flag, not after it
     load_particle_x(P, m.cap, p, x);
-    base_fx(m, x, base, fx);
+    act = P.active[p] != 0;
+    if (act) base_fx(m, x, base, fx);
   }
-  Box box;
-  if (!cta_box(m, act, base, box, sh)) return;
-  bool use_tile = box.vol <= kTileCap;
-  int off = 0;  // this thread's box in the tile
-  // The grid-updated velocities of a box, into the tile from `at`. Quotients of t < kTileCap by
-  // float reciprocals: (t + 1/2) / e is at least 1 / (2 e) from an integer, its rounding error
-  // below 2^-22 t / e.
-  auto stage = [&](const Box& b, int at) {
-    const int e12 = b.ext[1] * b.ext[2];
-    const float r12 = 1.f / (float)e12, r2 = 1.f / (float)b.ext[2];
-    for (int t = threadIdx.x; t < b.vol; t += blockDim.x) {
-      const int ti = (int)(((float)t + 0.5f) * r12), r = t - ti * e12;
-      const int tj = (int)(((float)r + 0.5f) * r2), tk = r - tj * b.ext[2];
-      const int i = b.lo[0] + ti, j = b.lo[1] + tj, k = b.lo[2] + tk;
-      float v[3];
-      grid_op(m, grid[node_index(m, i, j, k)], i, j, k, v);
-      tile[0][at + t] = v[0]; tile[1][at + t] = v[1]; tile[2][at + t] = v[2];
-    }
-  };
-  if (use_tile) {
-    stage(box, 0);
-  } else {
-    Box two[2];
-    const bool part = cut_boxes(m, act, base, two, sh, last);
-    use_tile = two[0].vol + two[1].vol <= kTileCap;
-    if (use_tile) {
-      stage(two[0], 0);
-      stage(two[1], two[0].vol);
-      box = part ? two[1] : two[0];
-      off = part ? two[0].vol : 0;
-    }
-  }
-  __syncthreads();
+  const Staged st = stage_stencils(m, act, base, tile, scratch, [&](int i, int j, int k, float v[3]) {
+    grid_op(m, grid[node_index(m, i, j, k)], i, j, k, v);
+  });
   if (!act) return;
-  if (use_tile) {
-    const int s1 = box.ext[2], s0 = box.ext[1] * s1;
-    const int t0 = off + (base[0] - box.lo[0]) * s0 + (base[1] - box.lo[1]) * s1 + (base[2] - box.lo[2]);
-    auto staged = [&](int i, int j, const bool*) {
-      return [tile, t = t0 + i * s0 + j * s1](int k, float v[3]) {
-        v[0] = tile[0][t + k]; v[1] = tile[1][t + k]; v[2] = tile[2][t + k];
-      };
-    };
+  if (st.ok) {
+    auto staged = [&](int i, int j, const bool*) { return [&st, i, j](int k, float v[3]) { st(i, j, k, v); }; };
     if (base[0] >= 0 && base[0] + 2 < m.nx && base[1] >= 0 && base[1] + 2 < m.ny && base[2] >= 0 &&
         base[2] + 2 < m.nz)
       g2p_gather<true>(m, P, p, base, fx, staged);
@@ -971,6 +1003,55 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
       };
     });
   }
+}
+
+// Inputs of coupling_particle loaded before the staging, so that its round trips to memory cover
+// theirs.
+struct CouplingInputs : Staged {
+  static constexpr int kBatch = 3;
+  float xs[3], vs[3], ms, vl;
+  uint32_t fl;
+  __device__ __forceinline__ float x(const ForceArgs&, int, int ax) const { return xs[ax]; }
+  __device__ __forceinline__ float v(const ForceArgs&, int, int ax) const { return vs[ax]; }
+  __device__ __forceinline__ float mass(const ForceArgs&, int) const { return ms; }
+  __device__ __forceinline__ float vol(const ForceArgs&, int) const { return vl; }
+  __device__ __forceinline__ uint32_t flag(const ForceArgs&, long long) const { return fl; }
+};
+
+// coupling_forces_body with the lattice velocities of the CTA's stencils staged in shared memory;
+// every thread calls it. tile: 3 x kTileCap floats of shared memory.
+// Read directly, each of the 27 loads of a warp takes 16 wavefronts (as in g2p_body) and the warps
+// wait on them: 88 us for 502,304 particles, 79 staged. What is left is the spread's 27 vector
+// reductions a particle (58 us without them) and the issue of some 2,000 instructions a
+// warp. The reductions stay one per particle and node: summed in runs first they would be fewer, but
+// 16-bit lattices amplify another order of that sum.
+__device__ __forceinline__ void coupling_staged_body(const ForceArgs& a, int p, float (*tile)[kTileCap],
+                                                     StageScratch& scratch) {
+  CouplingInputs in;
+  bool act = false;
+  in.ms = in.vl = 0.f;
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) in.xs[ax] = in.vs[ax] = 0.f;
+  if (p < a.n) {  // together, whether active or not
+    act = a.active[p] != 0;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) { in.xs[ax] = a.x[ax * a.cap + p]; in.vs[ax] = a.v[ax * a.cap + p]; }
+    in.ms = a.mass[p];
+    in.vl = a.vol[p];
+  }
+  int base[3] = {0, 0, 0};
+  float fx[3];
+  if (act) stencil_base(a.c.inv_dx, in.xs, base, fx);
+  in.fl = 0;
+  if (act && base[0] >= 0 && base[0] + 2 < a.g.nx && base[1] >= 0 && base[1] + 2 < a.g.ny && base[2] >= 0 &&
+      base[2] + 2 < a.g.nz)
+    in.fl = a.flags[((long long)(base[0] + 1) * a.g.ny + base[1] + 1) * a.g.nz + base[2] + 1];
+  static_cast<Staged&>(in) =
+      stage_stencils(a.g, act, base, tile, scratch, [&](int i, int j, int k, float v[3]) {
+        const float4 u = a.macro[((long long)i * a.g.ny + j) * a.g.nz + k];
+        v[0] = u.x; v[1] = u.y; v[2] = u.z;
+      });
+  coupling_forces_body<false>(a, p, in);
 }
 
 // The dirty ones of the 4^3 node blocks [b0, b0 + kBlock) (each of the CTA's kBlock threads looks
