@@ -6,9 +6,8 @@
 // thread scheduling:
 //   1. count:    per particle, its base cell's slot (atomic), its 8^3 cell tile's count and a
 //                mark on the node tiles its stencil touches.
-//   2. tiles:    a two-pass scan of the tile counts (tile starts); the non-empty cell tiles and
-//                the marked node tiles are listed, and counts and marks reset for the next
-//                substep.
+//   2. tiles:    a scan of the tile counts (tile starts); the non-empty cell tiles and the marked
+//                node tiles are listed, and the marks reset for the next substep.
 //   3. cells:    per non-empty tile, a block scans its 512 cell counts (cell starts) and lists
 //                its non-empty triples of cells along z.
 //   4. scatter:  per particle, its index into its cell's range (arrival order).
@@ -159,10 +158,53 @@ __global__ void __launch_bounds__(kBlock) sort_count_kernel(Mpm m, PView P, Sort
   }
 }
 
-// 2a. Per chunk of 1024 cell tiles: the exclusive prefix of the tile counts within the chunk
-// (into tile_start) and the chunk's total (into chunk_sum).
-__global__ void __launch_bounds__(kScanThreads) sort_tile_scan_local_kernel(SortGeo g, Work w) {
+// The tile start of cell tile i, and the tile in the list if it is not empty (arrival order: the
+// list only schedules work).
+__device__ __forceinline__ void put_tile(const SortGeo& g, const Work& w, int i, int count, int start) {
+  if (i >= g.ntiles) return;
+  w.tile_start[i] = start;
+  if (i == g.ntiles - 1) w.tile_start[g.ntiles] = start + count;
+  if (count > 0) w.cell_tiles[atomicAdd(&w.header[0], 1)] = i;
+}
+
+// The node tile i in the list if some stencil touched it (arrival order); its mark is reset.
+__device__ __forceinline__ void put_node_tile(const SortGeo& g, const Work& w, int i) {
+  if (i >= g.nntiles || w.node_flag[i] == 0) return;
+  w.node_flag[i] = 0;
+  w.node_tiles[atomicAdd(&w.header[1], 1)] = i;
+}
+
+// 2. Tile starts and lists in one launch: blocks [0, chunks) take 1024 cell tiles each and sum the
+// counts of all tiles before theirs themselves, the others 1024 node tiles each. (Up to
+// kDirectChunks chunks, 256 KB of counts: three launches of 1.3 to 1.8 us and the gaps between
+// them for one of 2.6 us: 9.64 -> 9.21 ms for 100 coupled substeps.)
+constexpr int kDirectChunks = 64;
+__global__ void __launch_bounds__(kScanThreads) sort_tiles_kernel(SortGeo g, Work w, int chunks) {
   __shared__ int ws[32];
+  if ((int)blockIdx.x >= chunks) {
+    put_node_tile(g, w, ((int)blockIdx.x - chunks) * kScanThreads + threadIdx.x);
+    return;
+  }
+  const int i0 = blockIdx.x * kScanThreads, i = i0 + threadIdx.x;
+  int before = 0;
+#pragma unroll 8
+  for (int t = threadIdx.x; t < i0; t += kScanThreads) before += w.tile_count[t];
+  const int c = i < g.ntiles ? w.tile_count[i] : 0;
+  int off, tot;
+  block_excl_scan(before, ws, &off);
+  const int ex = block_excl_scan(c, ws, &tot);
+  put_tile(g, w, i, c, off + ex);
+}
+
+// 2, larger grids. Per chunk of 1024 cell tiles: the exclusive prefix of the tile counts within
+// the chunk (into tile_start) and the chunk's total (into chunk_sum); the blocks past the chunks
+// take the node tiles.
+__global__ void __launch_bounds__(kScanThreads) sort_tile_scan_local_kernel(SortGeo g, Work w, int chunks) {
+  __shared__ int ws[32];
+  if ((int)blockIdx.x >= chunks) {
+    put_node_tile(g, w, ((int)blockIdx.x - chunks) * kScanThreads + threadIdx.x);
+    return;
+  }
   const int i = blockIdx.x * kScanThreads + threadIdx.x;
   const int c = i < g.ntiles ? w.tile_count[i] : 0;
   int tot;
@@ -171,36 +213,18 @@ __global__ void __launch_bounds__(kScanThreads) sort_tile_scan_local_kernel(Sort
   if (threadIdx.x == 0) w.chunk_sum[blockIdx.x] = tot;
 }
 
-// 2b. Tile starts = chunk offset + local prefix (the last block also writes the total); the
-// non-empty cell tiles are listed in arrival order (the list only schedules work) and the
-// tile counts reset.
+// Tile starts = chunk offset + local prefix.
 __global__ void __launch_bounds__(kScanThreads) sort_tile_scan_global_kernel(SortGeo g, Work w) {
-  __shared__ int off;
-  if (threadIdx.x == 0) {
-    int o = 0;
-    for (int b = 0; b < (int)blockIdx.x; ++b) o += w.chunk_sum[b];
-    off = o;
-    if (blockIdx.x == gridDim.x - 1) w.tile_start[g.ntiles] = o + w.chunk_sum[blockIdx.x];
-  }
-  __syncthreads();
+  __shared__ int ws[32];
+  int before = 0, off;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) before += w.chunk_sum[b];
+  block_excl_scan(before, ws, &off);
   const int i = blockIdx.x * kScanThreads + threadIdx.x;
-  if (i >= g.ntiles) return;
-  const int c = w.tile_count[i];
-  w.tile_start[i] += off;
-  if (c > 0) w.cell_tiles[atomicAdd(&w.header[0], 1)] = i;
-  w.tile_count[i] = 0;
-}
-
-// 2c. The node tiles some stencil touched are listed (arrival order) and their marks reset.
-__global__ void __launch_bounds__(kBlock) sort_node_tiles_kernel(SortGeo g, Work w) {
-  const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= g.nntiles || w.node_flag[i] == 0) return;
-  w.node_flag[i] = 0;
-  w.node_tiles[atomicAdd(&w.header[1], 1)] = i;
+  if (i < g.ntiles) put_tile(g, w, i, w.tile_count[i], w.tile_start[i] + off);
 }
 
 // 3. Cell starts (and the first sorted position of each non-empty cell) of each non-empty
-// cell tile, one block of 512 threads per tile; the cell counts are reset. The non-empty
+// cell tile, one block of 512 threads per tile; the cell and tile counts are reset. The non-empty
 // triples of cells (cells 0-2, 3-5 and 6-7 of a row of eight along z) are listed for the
 // partials, in arrival order (the list only schedules work; it has at most one entry per
 // particle).
@@ -218,6 +242,7 @@ __global__ void __launch_bounds__(kTC) sort_cell_scan_kernel(Work w) {
     w.cell_start[idx] = start;
     w.cell_row[idx] = c > 0 ? start : -1;
     w.cell_count[idx] = 0;
+    if (threadIdx.x == 0) w.tile_count[t] = 0;
     // a warp holds four rows; the first lane of a triple speaks for it
     const int z = lane & (kT - 1), cells = z == 6 ? 2 : 3;
     const int end = start + c;
@@ -614,7 +639,7 @@ int check_workspace(const Mpm& m, void* work, int64_t work_bytes, SortGeo& g, Wo
   return FSI_OK;
 }
 
-// The ten launches of a sorted substep (kCoupled: with the coupling folded in).
+// The eight launches of a sorted substep (kCoupled: with the coupling folded in).
 template <bool kCoupled>
 int sorted_substep(const Mpm& m, const PView& P, const SortGeo& g, const Work& w, float4* grid,
                    const ForceArgs& fa, cudaStream_t s) {
@@ -624,12 +649,16 @@ int sorted_substep(const Mpm& m, const PView& P, const SortGeo& g, const Work& w
   sort_count_kernel<<<pg, kBlock, 0, s>>>(m, P, g, w, kCoupled ? fa.cnt : nullptr);
   if (int e = check_launch("sort_count_kernel")) return e;
   const unsigned chunks = (unsigned)((g.ntiles + kScanThreads - 1) / kScanThreads);
-  sort_tile_scan_local_kernel<<<chunks, kScanThreads, 0, s>>>(g, w);
-  if (int e = check_launch("sort_tile_scan_local_kernel")) return e;
-  sort_tile_scan_global_kernel<<<chunks, kScanThreads, 0, s>>>(g, w);
-  if (int e = check_launch("sort_tile_scan_global_kernel")) return e;
-  sort_node_tiles_kernel<<<grid_for(g.nntiles, kBlock), kBlock, 0, s>>>(g, w);
-  if (int e = check_launch("sort_node_tiles_kernel")) return e;
+  const unsigned tile_blocks = chunks + (unsigned)((g.nntiles + kScanThreads - 1) / kScanThreads);
+  if (chunks <= kDirectChunks) {
+    sort_tiles_kernel<<<tile_blocks, kScanThreads, 0, s>>>(g, w, (int)chunks);
+    if (int e = check_launch("sort_tiles_kernel")) return e;
+  } else {
+    sort_tile_scan_local_kernel<<<tile_blocks, kScanThreads, 0, s>>>(g, w, (int)chunks);
+    if (int e = check_launch("sort_tile_scan_local_kernel")) return e;
+    sort_tile_scan_global_kernel<<<chunks, kScanThreads, 0, s>>>(g, w);
+    if (int e = check_launch("sort_tile_scan_global_kernel")) return e;
+  }
   sort_cell_scan_kernel<<<g.ntiles < 4 * sms ? g.ntiles : 4 * sms, kTC, 0, s>>>(w);
   if (int e = check_launch("sort_cell_scan_kernel")) return e;
   sort_scatter_kernel<<<pg, kBlock, 0, s>>>(m.n, w);
