@@ -7,6 +7,7 @@
 // reproduces each lattice's standalone run bit for bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -39,6 +40,7 @@ struct fsi_batch {
   fsi::Tile* ctiles = nullptr;      // device: (scene, first node block of kBlock)
   int nptiles = 0;
   int nctiles = 0;
+  bool even_cells = false;      // every lattice has an even number of cells
   long long capacity = 0;
   std::vector<fsi::BatchSolid> host_sol;
 };
@@ -329,6 +331,7 @@ extern "C" int fsi_batch_create(const fsi_batch_lattice* lattices, int32_t count
   b->storage = storage;
   b->arithmetic = arithmetic;
   b->cells = off;
+  b->even_cells = std::all_of(host.begin(), host.end(), [](const BatchLattice& L) { return L.g.n % 2 == 0; });
   if (cudaMalloc(&b->lat, sizeof(BatchLattice) * count) != cudaSuccess ||
       cudaMalloc(&b->tiles, sizeof(Tile) * tiles.size()) != cudaSuccess ||
       cudaMemcpy(b->lat, host.data(), sizeof(BatchLattice) * count, cudaMemcpyHostToDevice) !=
@@ -399,15 +402,15 @@ extern "C" int fsi_batch_lbm_step(const fsi_batch* b, void* pops, float* macro, 
   switch (b->storage) {
     case FSI_STORAGE_F16:
       return batch_step_launch_f16(b->lat, b->step_tiles, b->nstep_tiles, b->step_tile_cells,
-                                   b->variant, fast, odd, recompute, pops, macro, force,
+                                   b->variant, fast, odd, recompute, b->even_cells, pops, macro, force,
                                    force_prev, flags, s);
     case FSI_STORAGE_BF16:
       return batch_step_launch_bf16(b->lat, b->step_tiles, b->nstep_tiles, b->step_tile_cells,
-                                    b->variant, fast, odd, recompute, pops, macro, force,
+                                    b->variant, fast, odd, recompute, b->even_cells, pops, macro, force,
                                     force_prev, flags, s);
     default:
       return batch_step_launch_f32(b->lat, b->step_tiles, b->nstep_tiles, b->step_tile_cells,
-                                   b->variant, fast, odd, recompute, pops, macro, force,
+                                   b->variant, fast, odd, recompute, b->even_cells, pops, macro, force,
                                    force_prev, flags, s);
   }
 }

@@ -15,6 +15,7 @@ struct BatchStepArgs {
   const float* force;
   const float* force_prev;
   const uint32_t* flags;
+  bool pairs;  // every lattice has an even number of cells, the arrays are aligned (even_pairs)
 };
 
 // Minimum resident blocks per SM of register-cap variant kVar (0..2), 1 being the default.
@@ -29,8 +30,9 @@ constexpr int batch_min_blocks() {
 }
 
 // kStepBlock threads cover a tile of reps * kStepBlock * lanes cells: the exact form takes
-// one cell per thread and pass, the fast forms two (the packed lanes).
-template <int kStore, bool kFast, bool kOdd, bool kRecompute, int kVar>
+// one cell per thread and pass, the fast forms two (the packed lanes; kPairs: neighbours in memory,
+// on even steps of lattices that allow it, see step_even_pair).
+template <int kStore, bool kFast, bool kOdd, bool kRecompute, int kVar, bool kPairs>
 __global__ void __launch_bounds__(kStepBlock, (batch_min_blocks<kFast, kOdd, kRecompute, kVar>()))
     batch_step_kernel(BatchStepArgs b) {
   constexpr int NL = StepLanes<kFast>::n;
@@ -42,6 +44,11 @@ __global__ void __launch_bounds__(kStepBlock, (batch_min_blocks<kFast, kOdd, kRe
   __syncthreads();
   const LatticeView v = view_of<kStore>(L, rates, b.pops, b.macro, b.force, b.force_prev, b.flags);
   for (int r = 0; r < kReps; ++r) {
+    if constexpr (kPairs) {
+      const uint32_t c = 2 * (uint32_t)(t.first + r * kStepBlock + threadIdx.x);
+      if (c < (uint32_t)L.g.n) step_even_pair<kStore, kRecompute, LatticeView>(v, c);
+      continue;
+    }
     int ci[NL], cj[NL], ck[NL];
     bool has[NL];
     if (step_unit<NL>(L.g, (long long)t.first + r * kStepBlock + threadIdx.x, ci, cj, ck, has))
@@ -51,12 +58,19 @@ __global__ void __launch_bounds__(kStepBlock, (batch_min_blocks<kFast, kOdd, kRe
 
 template <int S, bool F, int V>
 void launch_variant(const BatchStepArgs& a, int ntiles, bool odd, bool recompute, cudaStream_t s) {
+  if constexpr (F) {
+    if (!odd && a.pairs) {
+      if (recompute) batch_step_kernel<S, F, false, true, V, true><<<ntiles, kStepBlock, 0, s>>>(a);
+      else batch_step_kernel<S, F, false, false, V, true><<<ntiles, kStepBlock, 0, s>>>(a);
+      return;
+    }
+  }
   if (recompute) {
-    if (odd) batch_step_kernel<S, F, true, true, V><<<ntiles, kStepBlock, 0, s>>>(a);
-    else batch_step_kernel<S, F, false, true, V><<<ntiles, kStepBlock, 0, s>>>(a);
+    if (odd) batch_step_kernel<S, F, true, true, V, false><<<ntiles, kStepBlock, 0, s>>>(a);
+    else batch_step_kernel<S, F, false, true, V, false><<<ntiles, kStepBlock, 0, s>>>(a);
   } else {
-    if (odd) batch_step_kernel<S, F, true, false, V><<<ntiles, kStepBlock, 0, s>>>(a);
-    else batch_step_kernel<S, F, false, false, V><<<ntiles, kStepBlock, 0, s>>>(a);
+    if (odd) batch_step_kernel<S, F, true, false, V, false><<<ntiles, kStepBlock, 0, s>>>(a);
+    else batch_step_kernel<S, F, false, false, V, false><<<ntiles, kStepBlock, 0, s>>>(a);
   }
 }
 
@@ -71,11 +85,12 @@ void launch_form(const BatchStepArgs& a, int ntiles, int variant, bool odd, bool
 }  // namespace
 
 int FSI_BATCH_STEP_NAME(const void* lat, const void* tiles, int ntiles, int tile_cells,
-                        int variant, bool fast, bool odd, bool recompute, void* pops,
+                        int variant, bool fast, bool odd, bool recompute, bool even_cells, void* pops,
                         float* macro, const float* force, const float* force_prev,
                         const uint32_t* flags, cudaStream_t stream) {
   BatchStepArgs a{static_cast<const BatchLattice*>(lat), static_cast<const Tile*>(tiles), 0,
-                  pops, macro, force, force_prev, flags};
+                  pops, macro, force, force_prev, flags,
+                  even_cells && even_pairs(0, pops, flags, force, force_prev)};
   a.reps = tile_cells / (kStepBlock * (fast ? 2 : 1));
 #if FSI_BATCH_STEP_STORAGE == FSI_STORAGE_F32
   if (fast) launch_form<FSI_STORAGE_F32, true>(a, ntiles, variant, odd, recompute, stream);

@@ -224,15 +224,15 @@ struct PersistArgs {
 // lat / tiles: device tables; tile_cells: cells per step tile (a multiple of 128, or of 256
 // for the fast forms); variant: register-cap variant 0..2.
 int batch_step_launch_f32(const void* lat, const void* tiles, int ntiles, int tile_cells,
-                          int variant, bool fast, bool odd, bool recompute, void* pops,
+                          int variant, bool fast, bool odd, bool recompute, bool even_cells, void* pops,
                           float* macro, const float* force, const float* force_prev,
                           const uint32_t* flags, cudaStream_t stream);
 int batch_step_launch_f16(const void* lat, const void* tiles, int ntiles, int tile_cells,
-                          int variant, bool fast, bool odd, bool recompute, void* pops,
+                          int variant, bool fast, bool odd, bool recompute, bool even_cells, void* pops,
                           float* macro, const float* force, const float* force_prev,
                           const uint32_t* flags, cudaStream_t stream);
 int batch_step_launch_bf16(const void* lat, const void* tiles, int ntiles, int tile_cells,
-                           int variant, bool fast, bool odd, bool recompute, void* pops,
+                           int variant, bool fast, bool odd, bool recompute, bool even_cells, void* pops,
                            float* macro, const float* force, const float* force_prev,
                            const uint32_t* flags, cudaStream_t stream);
 

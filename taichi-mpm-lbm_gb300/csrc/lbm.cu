@@ -364,6 +364,14 @@ void dispatch_forms(const fsi_lbm_desc* d, Args&&... args) {
 template <int S, bool F>
 struct StepLauncher {
   static void run(const StepArgs& a, bool odd, bool recompute, const CellLaunch& L, cudaStream_t s) {
+    if constexpr (F) {
+      if (!odd && even_pairs(a.g.n, a.pops, a.flags, a.force, a.force_prev)) {
+        const unsigned blocks = grid_for(a.g.n / 2, kStepBlock);
+        if (recompute) lbm_even_pair_kernel<S, true><<<blocks, kStepBlock, 0, s>>>(a);
+        else lbm_even_pair_kernel<S, false><<<blocks, kStepBlock, 0, s>>>(a);
+        return;
+      }
+    }
     if (recompute) {
       if (odd) lbm_step_kernel<S, F, true, true><<<L.grid, L.block, 0, s>>>(a);
       else lbm_step_kernel<S, F, false, true><<<L.grid, L.block, 0, s>>>(a);
