@@ -69,6 +69,30 @@ __global__ void __launch_bounds__(kTileCells)
   }
 }
 
+// The same in the fast form, two neighbouring cells per thread (lattices with even numbers of cells).
+template <int kStore, bool kOddState>
+__global__ void __launch_bounds__(kTileCells / 2)
+    batch_macro_pair_kernel(const BatchLattice* __restrict__ lat, const Tile* __restrict__ tiles,
+                            const void* pops_v, const float* __restrict__ force_all,
+                            const uint32_t* __restrict__ flags_all, float* macro_all,
+                            double* __restrict__ diag) {
+  const Tile t = tiles[blockIdx.x];
+  const BatchLattice& L = lat[t.lattice];
+  const uint32_t c = (uint32_t)t.first + 2 * threadIdx.x;
+  float mass[2] = {0.f, 0.f}, vmax[2] = {0.f, 0.f};
+  if (c < (uint32_t)L.g.n)
+    macro_pair<kStore, kOddState>(
+        L.g, reinterpret_cast<const typename Store<kStore>::T*>(pops_v) + 19 * L.off, force_all + 3 * L.off,
+        flags_all + L.off, c, shifts_of(L), L.rho0, reinterpret_cast<float4*>(macro_all) + L.off, mass, vmax);
+  if (diag) {
+    for (int l = 0; l < 2; ++l) {
+      if (l > 0) __syncthreads();  // the first sums' shared scratch is no longer read
+      const float s[1] = {mass[l]};
+      block_accumulate<1>(diag + 2 * t.lattice, s, diag + 2 * t.lattice + 1, vmax[l]);
+    }
+  }
+}
+
 template <int kStore>
 __global__ void __launch_bounds__(kTileCells)
     batch_distribution_kernel(const BatchLattice* __restrict__ lat, const Tile* __restrict__ tiles,
@@ -146,6 +170,17 @@ template <int S, bool F>
 struct BatchMacroLauncher {
   static void run(const fsi_batch* b, const void* pops, const float* force, const uint32_t* flags,
                   int parity, float* macro, double* diag, cudaStream_t s) {
+    if constexpr (F) {
+      if (macro_by_pairs<S>(parity != 0) && b->even_cells && even_pairs(0, pops, flags, force, nullptr)) {
+        if (parity)
+          batch_macro_pair_kernel<S, true>
+              <<<b->ntiles, kTileCells / 2, 0, s>>>(b->lat, b->tiles, pops, force, flags, macro, diag);
+        else
+          batch_macro_pair_kernel<S, false>
+              <<<b->ntiles, kTileCells / 2, 0, s>>>(b->lat, b->tiles, pops, force, flags, macro, diag);
+        return;
+      }
+    }
     batch_macro_kernel<S, F><<<b->ntiles, kTileCells, 0, s>>>(b->lat, b->tiles, pops, force, flags,
                                                               parity, macro, diag);
   }

@@ -155,6 +155,22 @@ __global__ void __launch_bounds__(kBlock) lbm_macro_kernel(MacroArgs a, double* 
   }
 }
 
+template <int kStore, bool kOddState>
+__global__ void __launch_bounds__(kBlock) lbm_macro_pair_kernel(MacroArgs a, double* __restrict__ diag) {
+  const uint32_t c = 2 * (blockIdx.x * kBlock + threadIdx.x);
+  float mass[2] = {0.f, 0.f}, vmax[2] = {0.f, 0.f};
+  if (c < (uint32_t)a.g.n)
+    macro_pair<kStore, kOddState>(a.g, reinterpret_cast<const typename Store<kStore>::T*>(a.pops), a.force,
+                                  a.flags, c, a.shift, a.rho0, a.macro, mass, vmax);
+  if (diag) {
+    for (int l = 0; l < 2; ++l) {
+      if (l > 0) __syncthreads();  // the first sums' shared scratch is no longer read
+      const float s[1] = {mass[l]};
+      block_accumulate<1>(diag, s, diag + 1, vmax[l]);
+    }
+  }
+}
+
 template <int kStore>
 __global__ void __launch_bounds__(kBlock) lbm_distribution_kernel(LbmGeom g, const void* pops_v,
                                                                   const uint32_t* __restrict__ flags,
@@ -385,6 +401,14 @@ struct StepLauncher {
 template <int S, bool F>
 struct MacroLauncher {
   static void run(const MacroArgs& a, double* diag, cudaStream_t s) {
+    if constexpr (F) {
+      if (macro_by_pairs<S>(a.parity != 0) && even_pairs(a.g.n, a.pops, a.flags, a.force, nullptr)) {
+        const unsigned blocks = grid_for(a.g.n / 2, kBlock);
+        if (a.parity) lbm_macro_pair_kernel<S, true><<<blocks, kBlock, 0, s>>>(a, diag);
+        else lbm_macro_pair_kernel<S, false><<<blocks, kBlock, 0, s>>>(a, diag);
+        return;
+      }
+    }
     const CellLaunch L = cell_launch(a.g);
     lbm_macro_kernel<S, F><<<L.grid, L.block, 0, s>>>(a, diag);
   }

@@ -91,3 +91,51 @@ def test_batch_pairs_equal_rows(storage, recompute):
     (p0, m0), (p1, m1) = _both_ways(call, batch._pops, batch._macro, force, prev)
     assert not torch.equal(p0, batch._pops)
     assert torch.equal(p0, p1) and torch.equal(m0, m1)
+
+
+@pytest.mark.parametrize("steps", [4, 5])
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_macro_pairs_equal_cells(shape, storage, steps):
+    """rho and u by pairs in both states of the populations; the diagnostic sums are float32 within a
+    warp (32 terms of either path, 32 u = 2e-6) and float64 across warps."""
+    rng = np.random.default_rng(shape[2])
+    lbm = LBMSolver3D(_config(shape, storage))
+    lbm.initialize((rng.uniform(size=shape) < 0.3).astype(np.int32))
+    for _ in range(steps):
+        lbm.step()
+    force = lbm._force_buf[lbm._fcur]
+    out = []
+    for f in (force, _mid_pair(force)):
+        m, diag = torch.full_like(lbm._macro, -1.0), torch.zeros(2, dtype=torch.float64, device="cuda")
+        plain = m.clone()
+        lbm._call("fsi_lbm_update_macro", nat.ptr(lbm._pops), nat.ptr(f), nat.ptr(lbm._flags), steps,
+                  nat.ptr(plain), nat.stream_ptr())
+        lbm._call("fsi_lbm_macro_diagnostics", nat.ptr(lbm._pops), nat.ptr(f), nat.ptr(lbm._flags), steps,
+                  nat.ptr(m), nat.ptr(diag), nat.stream_ptr())
+        assert torch.equal(m, plain)
+        out.append((m, diag))
+    (m0, d0), (m1, d1) = out
+    assert torch.equal(m0, m1)
+    assert d0[1] == d1[1] and abs(d0[0] / d1[0] - 1) < 4e-6
+
+
+@pytest.mark.parametrize("steps", [4, 5])
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+def test_batch_macro_pairs_equal_cells(storage, steps):
+    rng = np.random.default_rng(3)
+    batch = LatticeBatch([_config(s, storage) for s in SHAPES])
+    batch.initialize([(rng.uniform(size=s) < 0.3).astype(np.int32) for s in SHAPES])
+    for _ in range(steps):
+        batch.step()
+    force = batch._force_buf[batch._fcur]
+    out = []
+    for f in (force, _mid_pair(force)):
+        m = torch.full_like(batch._macro, -1.0)
+        diag = torch.zeros((len(SHAPES), 2), dtype=torch.float64, device="cuda")
+        nat.call("fsi_batch_lbm_macro", batch._handle, nat.ptr(batch._pops), nat.ptr(f), nat.ptr(batch._flags),
+                 steps, nat.ptr(m), nat.ptr(diag), nat.stream_ptr())
+        out.append((m, diag))
+    (m0, d0), (m1, d1) = out
+    assert torch.equal(m0, m1)
+    assert torch.equal(d0[:, 1], d1[:, 1]) and float((d0[:, 0] / d1[:, 0] - 1).abs().max()) < 4e-6
