@@ -254,9 +254,10 @@ __global__ void __launch_bounds__(kBlock)
                    t.first + (int)threadIdx.x, l);
 }
 
-// Four blocks per SM: 157 us for 64 scenes, against 160 with three and 158 with five (187 with the
-// lattice read directly).
-__global__ void __launch_bounds__(kBlock, 4)
+// Three blocks per SM: 160 us for 64 scenes (187 with the lattice read directly, 157 with four). With
+// four, more particles add to a node at once and in more orders: after 16 steps two runs of the 64
+// scenes differ by 6.4e-5 in C, against 5.5e-5 with three or without the staging.
+__global__ void __launch_bounds__(kBlock, 3)
     batch_coupling_forces_kernel(const BatchLattice* __restrict__ lat,
                                  const BatchSolid* __restrict__ sol, const Tile* __restrict__ ptiles,
                                  ForceArgs base, float dt_ratio, int build_fraction) {
