@@ -173,8 +173,8 @@ typedef struct fsi_mpm_desc {
   float clamp_upper[3];
   int32_t material; /* FSI_MATERIAL_*; the reference's model is fixed-corotated */
   /* Launch tuning of the tiled scatter (no reference counterpart; fsi.autotune sets them):
-   * threads per block of P2G and G2P, 128, 256 or 512 (0: 256), which sets the particles whose
-   * stencils share one shared-memory tile; and where a coupled tiled substep forms the
+   * threads per block of P2G and G2P, 128, 256 or 512 (0: 256), which sets the particles that
+   * P2G sorts and sums together and whose stencils G2P stages together; and where a coupled tiled substep forms the
    * coupling force: 0 by particle count, 1 inside P2G, 2 in a kernel of its own first, 3 in
    * a force kernel and a spread kernel of their own first. */
   int32_t launch_threads;
@@ -233,7 +233,7 @@ int fsi_mpm_substep_noalloc(const fsi_mpm_desc* desc, const fsi_particles* parti
 
 /* Bytes of the workspace that fsi_mpm_substep_sorted and fsi_coupled_substep need for this
  * grid and a particle capacity: the per-cell and per-tile counts and starts of the particle
- * sort, the sorted order and a 128-byte record per particle. The workspace is one device
+ * sort, the sorted order, a 16-byte list entry and a 128-byte record per particle. The workspace is one device
  * buffer, 256-byte aligned and zero-filled once before its first use; the substeps leave its
  * count arrays zero again. No reference counterpart (the reference does not sort). */
 int fsi_mpm_workspace_bytes(const fsi_mpm_desc* desc, int64_t capacity, int64_t* bytes);
@@ -490,7 +490,8 @@ int fsi_batch_destroy(fsi_batch* batch);
 int fsi_batch_cells(const fsi_batch* batch, int64_t* cells);
 
 /* Launch parameters of the batched lattice step, chosen by a caller's autotuner: cells per
- * thread block (a multiple of 128, or of 256 for the fast forms; default 256) and the
+ * thread block (a multiple of 128, or of 256 for the fast forms; default the widest of 1024, 512
+ * and 256 that gives four waves of blocks) and the
  * register-cap variant 0..2 (default 1). The exact form's results do not depend on them; the
  * fast forms' may differ in the last bits (the assembler schedules each variant apart). */
 int fsi_batch_tune(fsi_batch* batch, int32_t step_tile_cells, int32_t variant);
