@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock)
   auto& sm = *reinterpret_cast<ScatterSmem<kBlock>*>(scatter_smem);
   const Tile t = ptiles[blockIdx.x];
   const Mpm m = sol[t.lattice].m;
-  p2g_runs_body<kBlock>(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
+  p2g_runs_body<kBlock, false>(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
                         t.first * kBlock + threadIdx.x, sm);
 }
 
@@ -254,9 +254,10 @@ __global__ void __launch_bounds__(kBlock)
                    t.first + (int)threadIdx.x, l);
 }
 
-// Three blocks per SM: 160 us for 64 scenes (187 with the lattice read directly, 157 with four). With
-// four, more particles add to a node at once and in more orders: after 16 steps two runs of the 64
-// scenes differ by 6.4e-5 in C, against 5.5e-5 with three or without the staging.
+// Three blocks per SM: 187 us for 64 scenes, against 212 at its natural 101 registers (two) and 210
+// at 64 (four, spills). With the lattice velocities staged as coupling_only_kernel does it takes 160
+// (157 with four blocks), but then a block's warps add to the accumulator together, in more orders:
+// two runs of 64 FP16 scenes differ by 6.6 to 7.4e-5 in C after a second pass of 8 steps, against 6.0e-5.
 __global__ void __launch_bounds__(kBlock, 3)
     batch_coupling_forces_kernel(const BatchLattice* __restrict__ lat,
                                  const BatchSolid* __restrict__ sol, const Tile* __restrict__ ptiles,
@@ -264,9 +265,7 @@ __global__ void __launch_bounds__(kBlock, 3)
   const Tile t = ptiles[blockIdx.x];
   const ForceArgs a = scene_force_args(base, lat[t.lattice], sol[t.lattice], t.lattice, dt_ratio,
                                        build_fraction);
-  __shared__ float tile[3][kTileCap];
-  __shared__ StageScratch scratch;
-  coupling_staged_body(a, t.first * kBlock + threadIdx.x, tile, scratch);
+  coupling_forces_body<false>(a, t.first * kBlock + threadIdx.x);
 }
 
 __global__ void __launch_bounds__(kTileCells)

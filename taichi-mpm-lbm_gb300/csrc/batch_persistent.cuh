@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
       for (int ti = blockIdx.x; ti < a.nptiles; ti += gridDim.x) {
         const Tile t = a.ptiles[ti];
         const BatchSolid& S = a.sol[t.lattice];
-        p2g_runs_body<kBlock>(S.m, a.P, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
+        p2g_runs_body<kBlock, false>(S.m, a.P, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
                               t.first * kBlock + threadIdx.x, p2g_smem);
         __syncthreads();  // the records are no longer read
       }

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(kT, 1024 / kT) p2g_kernel(Mpm m, PView P,
                                                             float4* __restrict__ grid,
                                                             uint8_t* __restrict__ dirty) {
   extern __shared__ float4 scatter_smem[];
-  p2g_runs_body<kT>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x,
+  p2g_runs_body<kT, true>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x,
                     *reinterpret_cast<ScatterSmem<kT>*>(scatter_smem));
 }
 
