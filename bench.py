@@ -41,7 +41,7 @@ COUPLED_BYTES_PER_PARTICLE = 224  # per particle-substep with the coupling force
 MPM_BYTES_PER_NODE = 32       # per touched grid node per substep
 # Kernel launches per call of each entry point the timed regions use.
 LAUNCHES = {"fsi_coupling_forces": 1, "fsi_mpm_substep": 3, "fsi_mpm_substep_sorted": 10,
-            "fsi_coupled_substep": 10, "fsi_coupled_substep_tiled": 4,
+            "fsi_coupled_substep": 10, "fsi_coupled_substep_tiled_storage": 4,
             "fsi_coupling_assemble": 1, "fsi_contact": 1,
             "fsi_lbm_update_macro": 1, "fsi_lbm_macro_diagnostics": 1, "fsi_lbm_reduce": 1,
             "fsi_coupled_diagnostics": 1, "fsi_lbm_force_op": 1, "fsi_mpm_reduce": 1,
@@ -83,7 +83,7 @@ def launches_since(before, lbm_step_launches: int = 1, tiled_substep_launches: i
     separate force and spread kernels)."""
     from fsi import _native as nat
     table = dict(LAUNCHES, fsi_lbm_step=lbm_step_launches,
-                 fsi_coupled_substep_tiled=tiled_substep_launches)
+                 fsi_coupled_substep_tiled_storage=tiled_substep_launches)
     total = 0
     for name, count in nat.CALLS.items():
         total += (count - before.get(name, 0)) * table.get(name, 1)

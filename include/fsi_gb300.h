@@ -337,6 +337,15 @@ int fsi_coupled_substep_tiled(const fsi_coupling_desc* coupling, const fsi_mpm_d
                               int32_t* coupling_mask, void* counters, float* grid,
                               uint8_t* dirty, void* stream);
 
+/* The same beside a lattice whose population storage (FSI_STORAGE_*) is known: launches of many
+ * particles beside an FP32 lattice sum in a faster order (fsi_coupled_substep_tiled sums as beside a
+ * 16-bit one, whose populations amplify a changed order of the reaction's sums). */
+int fsi_coupled_substep_tiled_storage(int32_t storage, const fsi_coupling_desc* coupling,
+                                      const fsi_mpm_desc* desc, const fsi_particles* particles,
+                                      const float* macro, const uint32_t* flags, float* accum,
+                                      float* valid_weight, int32_t* coupling_mask, void* counters,
+                                      float* grid, uint8_t* dirty, void* stream);
+
 /* Rebuilds the LBM force field float[3][N] for the next lattice step:
  *   FSI_ASSEMBLE_CLAMP_FRACTION  accum.w = min(accum.w, 1)   (coupling.py:408-411)
  *   (always)                     force = fluid ? base : 0     (lbm3d.py:504-510)

@@ -222,7 +222,7 @@ int check_batch(const fsi_batch* b) {
 // ------------------------------------------------------------------ solids
 
 // One CTA per (scene, block of kBlock particles): the single-solver P2G / G2P bodies on the
-// scene's grid block.
+// scene's grid block. P2G in runs, or through a tile of nodes beside 16-bit lattices (scatter_in_runs).
 __global__ void __launch_bounds__(kBlock, 1024 / kBlock)
     batch_p2g_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
                      const Tile* __restrict__ ptiles, PView P, float4* grid_all, uint8_t* dirty_all) {
@@ -230,8 +230,18 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock)
   auto& sm = *reinterpret_cast<ScatterSmem<kBlock>*>(scatter_smem);
   const Tile t = ptiles[blockIdx.x];
   const Mpm m = sol[t.lattice].m;
-  p2g_runs_body<kBlock, false>(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
+  p2g_runs_body<kBlock>(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
                         t.first * kBlock + threadIdx.x, sm);
+}
+
+__global__ void __launch_bounds__(kBlock)
+    batch_p2g_tile_kernel(const BatchLattice* __restrict__ lat, const BatchSolid* __restrict__ sol,
+                          const Tile* __restrict__ ptiles, PView P, float4* grid_all,
+                          uint8_t* dirty_all) {
+  const Tile t = ptiles[blockIdx.x];
+  const Mpm m = sol[t.lattice].m;
+  p2g_tile_body<false>(m, P, grid_all + lat[t.lattice].off, dirty_all + sol[t.lattice].block_off,
+                       t.first * kBlock + threadIdx.x, nullptr);
 }
 
 __global__ void __launch_bounds__(kBlock, 1280 / kBlock)
@@ -254,11 +264,8 @@ __global__ void __launch_bounds__(kBlock)
                    t.first + (int)threadIdx.x, l);
 }
 
-// Three blocks per SM: 187 us for 64 scenes, against 212 at its natural 101 registers (two) and 210
-// at 64 (four, spills). With the lattice velocities staged as coupling_only_kernel does it takes 160
-// (157 with four blocks), but then a block's warps add to the accumulator together, in more orders:
-// two runs of 64 FP16 scenes differ by 6.6 to 7.4e-5 in C after a second pass of 8 steps, against 6.0e-5.
-__global__ void __launch_bounds__(kBlock, 3)
+// The lattice read directly, beside 16-bit lattices (scatter_in_runs), at its natural 101 registers.
+__global__ void __launch_bounds__(kBlock)
     batch_coupling_forces_kernel(const BatchLattice* __restrict__ lat,
                                  const BatchSolid* __restrict__ sol, const Tile* __restrict__ ptiles,
                                  ForceArgs base, float dt_ratio, int build_fraction) {
@@ -266,6 +273,19 @@ __global__ void __launch_bounds__(kBlock, 3)
   const ForceArgs a = scene_force_args(base, lat[t.lattice], sol[t.lattice], t.lattice, dt_ratio,
                                        build_fraction);
   coupling_forces_body<false>(a, t.first * kBlock + threadIdx.x);
+}
+
+// The lattice velocities staged, as in coupling_only_kernel: 157 us for 64 scenes, against 212.
+__global__ void __launch_bounds__(kBlock, 4)
+    batch_coupling_staged_kernel(const BatchLattice* __restrict__ lat,
+                                 const BatchSolid* __restrict__ sol, const Tile* __restrict__ ptiles,
+                                 ForceArgs base, float dt_ratio, int build_fraction) {
+  __shared__ float tile[3][kTileCap];
+  __shared__ StageScratch scratch;
+  const Tile t = ptiles[blockIdx.x];
+  const ForceArgs a = scene_force_args(base, lat[t.lattice], sol[t.lattice], t.lattice, dt_ratio,
+                                       build_fraction);
+  coupling_staged_body(a, t.first * kBlock + threadIdx.x, tile, scratch);
 }
 
 __global__ void __launch_bounds__(kTileCells)
@@ -595,9 +615,13 @@ extern "C" int fsi_batch_mpm_substep(const fsi_batch* b, const fsi_particles* pa
   if (b->nptiles == 0) return FSI_OK;
   cudaStream_t s = as_stream(stream);
   float4* g4 = reinterpret_cast<float4*>(grid);
-  constexpr size_t smem = sizeof(ScatterSmem<kBlock>);
-  if (int e = opt_in_smem<batch_p2g_kernel>((int)smem)) return e;
-  batch_p2g_kernel<<<b->nptiles, kBlock, smem, s>>>(b->lat, b->sol, b->ptiles, P, g4, dirty);
+  if (scatter_in_runs(b->storage)) {
+    constexpr size_t smem = sizeof(ScatterSmem<kBlock>);
+    if (int e = opt_in_smem<batch_p2g_kernel>((int)smem)) return e;
+    batch_p2g_kernel<<<b->nptiles, kBlock, smem, s>>>(b->lat, b->sol, b->ptiles, P, g4, dirty);
+  } else {
+    batch_p2g_tile_kernel<<<b->nptiles, kBlock, 0, s>>>(b->lat, b->sol, b->ptiles, P, g4, dirty);
+  }
   if (int e = check_launch("batch_p2g_kernel")) return e;
   batch_g2p_kernel<<<b->nptiles, kBlock, 0, s>>>(b->lat, b->sol, b->ptiles, P, g4);
   if (int e = check_launch("batch_g2p_kernel")) return e;
@@ -624,8 +648,10 @@ extern "C" int fsi_batch_coupling_forces(const fsi_batch* b, const fsi_particles
   a.valid_out = valid_weight;
   a.mask_out = coupling_mask;
   a.cnt = reinterpret_cast<Cnt*>(counters);
-  batch_coupling_forces_kernel<<<b->nptiles, kBlock, 0, as_stream(stream)>>>(
-      b->lat, b->sol, b->ptiles, a, dt_ratio, build_fraction);
+  const auto kernel =
+      scatter_in_runs(b->storage) ? batch_coupling_staged_kernel : batch_coupling_forces_kernel;
+  kernel<<<b->nptiles, kBlock, 0, as_stream(stream)>>>(b->lat, b->sol, b->ptiles, a, dt_ratio,
+                                                       build_fraction);
   return check_launch("batch_coupling_forces_kernel");
 }
 

@@ -133,9 +133,13 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
       for (int ti = blockIdx.x; ti < a.nptiles; ti += gridDim.x) {
         const Tile t = a.ptiles[ti];
         const BatchSolid& S = a.sol[t.lattice];
-        p2g_runs_body<kBlock, false>(S.m, a.P, a.grid + a.lat[t.lattice].off, a.dirty + S.block_off,
-                              t.first * kBlock + threadIdx.x, p2g_smem);
-        __syncthreads();  // the records are no longer read
+        float4* const grid = a.grid + a.lat[t.lattice].off;
+        const int p = t.first * kBlock + threadIdx.x;
+        if constexpr (kStore == FSI_STORAGE_F32)  // scatter_in_runs
+          p2g_runs_body<kBlock>(S.m, a.P, grid, a.dirty + S.block_off, p, p2g_smem);
+        else
+          p2g_tile_body<false, true>(S.m, a.P, grid, a.dirty + S.block_off, p, nullptr, tile);
+        __syncthreads();  // the block's shared memory is no longer read
       }
       if (!grid_barrier(a, epoch)) return;
       for (int ti = blockIdx.x; ti < a.nptiles; ti += gridDim.x) {
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(kBlock, FSI_PERSIST_MIN_BLOCKS) batch_persiste
 // when the launch could not be made (the kernel's own timeout shows in a->err).
 int FSI_BATCH_PERSIST_NAME(const void* args, bool fast, cudaStream_t stream) {
   const PersistArgs& a = *static_cast<const PersistArgs*>(args);
-  const size_t tile = sizeof(float) * 3 * kTileCap, runs = sizeof(ScatterSmem<kBlock>);
+  const size_t tile = sizeof(float) * 4 * kTileCap, runs = sizeof(ScatterSmem<kBlock>);
   const size_t smem = tile > runs ? tile : runs;
   auto launch = [&](auto kernel) -> int {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=

@@ -143,9 +143,10 @@ int one_step(fsi_ctx* c, double lbm_dt, const float* body_force, int n_substeps,
                                 c->b.valid_weight, c->b.coupling_mask, c->b.counters, c->grid,
                                 c->workspace, c->workspace_bytes, stream);
       else
-        e = fsi_coupled_substep_tiled(&d.coupling, &d.mpm, P, c->b.macro, c->b.flags,
-                                      c->b.accum, c->b.valid_weight, c->b.coupling_mask,
-                                      c->b.counters, c->grid, c->dirty, stream);
+        e = fsi_coupled_substep_tiled_storage(d.lbm.storage, &d.coupling, &d.mpm, P, c->b.macro,
+                                              c->b.flags, c->b.accum, c->b.valid_weight,
+                                              c->b.coupling_mask, c->b.counters, c->grid, c->dirty,
+                                              stream);
       if (e) return e;
     } else {
       if (int e = clear_particle_force(c, s)) return e;

@@ -79,9 +79,9 @@ constexpr uint32_t kAllUsable = (1u << 27) - 1u;
 
 // Where coupling_particle takes its inputs from: memory, as they are needed. ok: the stencil's
 // lattice velocities are at hand (operator()); kBatch: else this many of their loads go out
-// together.
+// together. kStages: whether ok is ever set.
 struct FromMemory {
-  static constexpr bool ok = false;
+  static constexpr bool ok = false, kStages = false;
   static constexpr int kBatch = 9;
   __device__ __forceinline__ void operator()(int, int, int, float*) const {}
   __device__ __forceinline__ float x(const ForceArgs& a, int p, int ax) const { return a.x[ax * a.cap + p]; }
@@ -308,7 +308,9 @@ __device__ __forceinline__ void coupling_forces_body(const ForceArgs& a, int p, 
             red_add_v4(a.accum + c, t.x, t.y, t.z, t.w);
           }
         };
-        if (usable == kAllUsable && a.c.cell_volume == 1.0f)
+        // A path of its own for whole stencils where the lattice velocities are staged; read
+        // directly the spread is paced by the loads, and its order of arrival stays as it is.
+        if (In::kStages && usable == kAllUsable && a.c.cell_volume == 1.0f)
           spread(std::true_type{});
         else
           spread(std::false_type{});

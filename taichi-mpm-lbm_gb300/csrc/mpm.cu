@@ -37,8 +37,16 @@ __global__ void __launch_bounds__(kT, 1024 / kT) p2g_kernel(Mpm m, PView P,
                                                             float4* __restrict__ grid,
                                                             uint8_t* __restrict__ dirty) {
   extern __shared__ float4 scatter_smem[];
-  p2g_runs_body<kT, true>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x,
+  p2g_runs_body<kT>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x,
                     *reinterpret_cast<ScatterSmem<kT>*>(scatter_smem));
+}
+
+// The same through a tile of nodes, beside 16-bit lattices (scatter_in_runs).
+template <int kT>
+__global__ void __launch_bounds__(kT, 1024 / kT) p2g_tile_kernel(Mpm m, PView P,
+                                                                 float4* __restrict__ grid,
+                                                                 uint8_t* __restrict__ dirty) {
+  p2g_tile_body<false>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x, nullptr);
 }
 
 // The penalty coupling alone (one thread per particle), before p2g_kernel on large launches. Four
@@ -47,6 +55,11 @@ __global__ void __launch_bounds__(kBlock, 4) coupling_only_kernel(ForceArgs fa) 
   __shared__ float tile[3][kTileCap];
   __shared__ StageScratch scratch;
   coupling_staged_body(fa, blockIdx.x * kBlock + threadIdx.x, tile, scratch);
+}
+
+// The same with the lattice read directly, beside 16-bit lattices (scatter_in_runs).
+__global__ void __launch_bounds__(kBlock) coupling_direct_kernel(ForceArgs fa) {
+  coupling_forces_body<false>(fa, blockIdx.x * kBlock + threadIdx.x);
 }
 
 // The coupling split in two lighter kernels: the force (gathers), then the spread (vector
@@ -65,7 +78,7 @@ __global__ void __launch_bounds__(kBlock) coupling_spread_kernel(ForceArgs fa) {
 template <int kT>
 __global__ void __launch_bounds__(kT) coupled_p2g_kernel(Mpm m, PView P, float4* __restrict__ grid,
                                                          uint8_t* __restrict__ dirty, ForceArgs fa) {
-  coupled_p2g_tile_body(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x, fa);
+  p2g_tile_body<true>(m, P, grid, dirty, blockIdx.x * kT + threadIdx.x, &fa);
 }
 
 template <int kT>
@@ -90,6 +103,14 @@ struct P2G {
     constexpr size_t b = sizeof(ScatterSmem<kT>);
     if (int e = opt_in_smem<p2g_kernel<kT>>((int)b)) return e;
     p2g_kernel<kT><<<g, kT, b, s>>>(m, P, grid, dirty);
+    return check_launch(what);
+  }
+};
+template <int kT>
+struct P2GTile {
+  static int run(unsigned g, cudaStream_t s, const char* what, Mpm m, PView P, float4* grid,
+                 uint8_t* dirty) {
+    p2g_tile_kernel<kT><<<g, kT, 0, s>>>(m, P, grid, dirty);
     return check_launch(what);
   }
 };
@@ -364,11 +385,13 @@ extern "C" int fsi_mpm_substep_noalloc(const fsi_mpm_desc* d, const fsi_particle
   return gather_and_clear(m, P, g4, dirty, s);
 }
 
-extern "C" int fsi_coupled_substep_tiled(const fsi_coupling_desc* c, const fsi_mpm_desc* d,
-                                         const fsi_particles* parts, const float* macro,
-                                         const uint32_t* flags, float* accum, float* valid_weight,
-                                         int32_t* coupling_mask, void* counters, float* grid,
-                                         uint8_t* dirty, void* stream) {
+extern "C" int fsi_coupled_substep_tiled_storage(int32_t storage, const fsi_coupling_desc* c,
+                                                 const fsi_mpm_desc* d, const fsi_particles* parts,
+                                                 const float* macro, const uint32_t* flags,
+                                                 float* accum, float* valid_weight,
+                                                 int32_t* coupling_mask, void* counters, float* grid,
+                                                 uint8_t* dirty, void* stream) {
+  FSI_REQUIRE(storage >= FSI_STORAGE_F32 && storage <= FSI_STORAGE_BF16, "unknown storage %d", storage);
   Mpm m;
   PView P;
   if (int e = make_mpm(d, parts, m, P)) return e;
@@ -401,18 +424,35 @@ extern "C" int fsi_coupled_substep_tiled(const fsi_coupling_desc* c, const fsi_m
   // so the coupling runs first on its own (measured on the 384x192x192 coupled step: 3.71 ms
   // separate against 3.93 ms fused). m.fold overrides the choice.
   const bool fold = m.fold == 1 || (m.fold == 0 && m.n < 2 * 152 * kBlock);
+  const bool runs = scatter_in_runs(storage);
   if (fold) {
     if (int e = launch_tiled<CoupledP2G>(m.threads, m, s, "coupled_p2g_kernel", m, P, g4, dirty, fa)) return e;
-  } else if (m.fold == 3) {
+    return gather_and_clear(m, P, g4, dirty, s);
+  }
+  if (m.fold == 3) {
     coupling_gather_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
     if (int e = check_launch("coupling_gather_kernel")) return e;
     coupling_spread_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
     if (int e = check_launch("coupling_spread_kernel")) return e;
-    if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel", m, P, g4, dirty)) return e;
-  } else {
+  } else if (runs) {
     coupling_only_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
     if (int e = check_launch("coupling_only_kernel")) return e;
-    if (int e = launch_tiled<P2G>(m.threads, m, s, "p2g_kernel", m, P, g4, dirty)) return e;
+  } else {
+    coupling_direct_kernel<<<grid_for(m.n, kBlock), kBlock, 0, s>>>(fa);
+    if (int e = check_launch("coupling_direct_kernel")) return e;
   }
+  if (int e = runs ? launch_tiled<P2G>(m.threads, m, s, "p2g_kernel", m, P, g4, dirty)
+                   : launch_tiled<P2GTile>(m.threads, m, s, "p2g_tile_kernel", m, P, g4, dirty))
+    return e;
   return gather_and_clear(m, P, g4, dirty, s);
+}
+
+// The lattice's storage is not known here: the order of sums that every form takes.
+extern "C" int fsi_coupled_substep_tiled(const fsi_coupling_desc* c, const fsi_mpm_desc* d,
+                                         const fsi_particles* parts, const float* macro,
+                                         const uint32_t* flags, float* accum, float* valid_weight,
+                                         int32_t* coupling_mask, void* counters, float* grid,
+                                         uint8_t* dirty, void* stream) {
+  return fsi_coupled_substep_tiled_storage(FSI_STORAGE_F16, c, d, parts, macro, flags, accum, valid_weight,
+                                           coupling_mask, counters, grid, dirty, stream);
 }

@@ -429,6 +429,14 @@ __device__ __forceinline__ int block_excl_scan(int v, int* ws, int* total) {
   return excl;
 }
 
+// Whether the scatter beside a lattice of this population storage sums in runs (p2g_runs_body, the
+// coupling staged), or in the order of the tile (p2g_tile_body, the coupling read directly). A 16-bit
+// lattice turns last-bit differences of the reaction into whole quanta of its populations, so the sums
+// that feed it keep their order: with runs, C of 6 to 24 FP16 scenes after 8 steps is 2.3e-5 from the
+// tile's, with the tile 1.7e-5 from itself. The tile costs 335 us for 64 scenes, runs 109. FP32
+// lattices pass the differences on as they are: 2.1e-5 against 1.4e-5, over 80 substeps.
+inline bool scatter_in_runs(int32_t storage) { return storage == FSI_STORAGE_F32; }
+
 // ------------------------------------------------- P2G of a CTA's particles, in runs
 //
 // The scatter sums what a CTA's particles add to a node before anything is added in global
@@ -634,10 +642,9 @@ __device__ __forceinline__ void mark_cells(const Mpm& m, uint8_t* __restrict__ d
 // P2G of particle p (this thread) within its CTA of kT threads, in runs; every thread calls it.
 // A CTA whose bounding box does not fit the sort (particles of two bodies far apart, or
 // scattered ones) adds each contribution straight into global memory.
-// kAlternate: odd lanes walk the stencil backwards where contributions are added singly. The two
-// particles of a sub-cell pair, which share a base cell, then add into different nodes at each step.
-// Not in batches: two runs of 64 FP16 scenes differ by 7.4e-5 in C with it, by 6.7e-5 without.
-template <int kT, bool kAlternate>
+// Odd lanes walk the stencil backwards where contributions are added singly: the two particles of
+// a sub-cell pair, which share a base cell, then add into different nodes at each step.
+template <int kT>
 __device__ __forceinline__ void p2g_runs_body(const Mpm& m, const PView& P, float4* __restrict__ grid,
                                               uint8_t* __restrict__ dirty, int p,
                                               ScatterSmem<kT>& sm) {
@@ -688,7 +695,7 @@ __device__ __forceinline__ void p2g_runs_body(const Mpm& m, const PView& P, floa
     return;
   }
   if (!in) return;
-  const bool rev = kAlternate && (threadIdx.x & 1) != 0;
+  const bool rev = (threadIdx.x & 1) != 0;
 #pragma unroll 1
   for (int t = 0; t < 27; ++t) {
     const int s = rev ? 26 - t : t;
@@ -710,20 +717,26 @@ __device__ __forceinline__ void p2g_runs_body(const Mpm& m, const PView& P, floa
   }
 }
 
-// P2G of particle p (this thread) within its CTA with the penalty coupling folded in
-// (_compute_coupling_forces_kernel, fsi/coupling.py:332-406); every thread of the CTA calls it.
-// The particle's coupling force is formed first (it is P2G's dt f term), and the fluid reaction
-// and solid fraction are spread into fa.accum beside the grid scatter, which goes to a tile of
-// nodes in shared memory. For launches of few particles only, where one launch less counts.
+// P2G of particle p (this thread) within its CTA through a tile of nodes in shared memory: every
+// term rounded like the reference's, one addition per node and CTA into global memory. Every thread
+// of the CTA calls it. It serves the launches whose sums have to stay as they are:
+// kCoupled: with the penalty coupling folded in (_compute_coupling_forces_kernel,
+// fsi/coupling.py:332-406), for launches of few particles only, where one launch less counts. The
+// particle's coupling force is formed first (it is P2G's dt f term), and the fluid reaction and solid
+// fraction are spread into fa->accum beside the grid scatter.
 // Its loop of 27 paced steps also fixes the order in which CTAs reach a node in practice: over 47
 // pairs of equal three-step runs of the 4,096-particle smoke scene the lattices were the same bit
 // for bit, against 15 pairs that differ when the coupling is a kernel of its own, and 3 to 14 of
 // 23 with P2G in runs here (which takes 12 to 15 us for this launch's 27).
-__device__ __forceinline__ void coupled_p2g_tile_body(const Mpm& m, const PView& P,
-                                                      float4* __restrict__ grid,
-                                                      uint8_t* __restrict__ dirty, int p,
-                                                      const ForceArgs& fa) {
-  __shared__ float tile[4][kTileCap];
+// Not kCoupled: beside 16-bit lattices (scatter_in_runs).
+// kExtTile: the tile is the caller's shared memory `ext` (4 x kTileCap floats).
+template <bool kCoupled, bool kExtTile = false>
+__device__ __forceinline__ void p2g_tile_body(const Mpm& m, const PView& P,
+                                              float4* __restrict__ grid,
+                                              uint8_t* __restrict__ dirty, int p,
+                                              const ForceArgs* fa, float (*ext)[kTileCap] = nullptr) {
+  __shared__ float own[kExtTile ? 1 : 4][kExtTile ? 1 : kTileCap];
+  float (*tile)[kTileCap] = kExtTile ? ext : reinterpret_cast<float (*)[kTileCap]>(own);
   __shared__ int sh[8];
   const long long cap = m.cap;
   const bool act = p < m.n && P.active[p] != 0;
@@ -734,12 +747,12 @@ __device__ __forceinline__ void coupled_p2g_tile_body(const Mpm& m, const PView&
   // coupling: in-grid fluid stencil nodes (bit 9i + 3j + k), valid weight, force, volume
   uint32_t usable = 0;
   float valid = 0.f, pf[3] = {0.f, 0.f, 0.f}, vp = 0.f;
-  {
+  if (kCoupled) {
     bool partial = false, clipped = false, unsupported = false;
     if (act) {
       int cb[3];
       float cw[3][3];
-      if (!coupling_particle<false>(fa, p, cb, cw, usable, valid, pf, partial, clipped,
+      if (!coupling_particle<false>(*fa, p, cb, cw, usable, valid, pf, partial, clipped,
                                     unsupported)) {
         usable = 0;
         pf[0] = pf[1] = pf[2] = 0.f;
@@ -748,9 +761,9 @@ __device__ __forceinline__ void coupled_p2g_tile_body(const Mpm& m, const PView&
     } else if (p < m.n) {
       P.fp[p] = 0.f; P.fp[cap + p] = 0.f; P.fp[2 * cap + p] = 0.f;
     }
-    warp_count(&fa.cnt->unsupported, unsupported);
-    warp_count(&fa.cnt->partial, partial);
-    warp_count(&fa.cnt->clipped, clipped);
+    warp_count(&fa->cnt->unsupported, unsupported);
+    warp_count(&fa->cnt->partial, partial);
+    warp_count(&fa->cnt->clipped, clipped);
   }
   if (act) {
     float x[3];
@@ -760,7 +773,7 @@ __device__ __forceinline__ void coupled_p2g_tile_body(const Mpm& m, const PView&
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       mv[a] = __fmul_rn(mass, P.v[a * cap + p]);
-      dtf[a] = __fmul_rn(m.dt, pf[a]);
+      dtf[a] = __fmul_rn(m.dt, kCoupled ? pf[a] : P.fp[a * cap + p]);
     }
   }
 
@@ -825,10 +838,10 @@ __device__ __forceinline__ void coupled_p2g_tile_body(const Mpm& m, const PView&
           }
           const float addm = __fmul_rn(w, mass);
           const long long t = t0 + oa[0][si] * st0 + oa[1][sj] * st1 + oa[2][sk];
-          if ((usable >> (9 * oa[0][si] + 3 * oa[1][sj] + oa[2][sk])) & 1u) {
-            float4 c = coupling_spread_terms(fa.c, w, valid, pf, vp);
-            if (!fa.c.build_fraction) c.w = 0.f;
-            red_add_v4(fa.accum + g0 + oa[0][si] * gs0 + oa[1][sj] * m.nz + oa[2][sk],
+          if (kCoupled && (usable >> (9 * oa[0][si] + 3 * oa[1][sj] + oa[2][sk])) & 1u) {
+            float4 c = coupling_spread_terms(fa->c, w, valid, pf, vp);
+            if (!fa->c.build_fraction) c.w = 0.f;
+            red_add_v4(fa->accum + g0 + oa[0][si] * gs0 + oa[1][sj] * m.nz + oa[2][sk],
                        c.x, c.y, c.z, c.w);
           }
           if (use_tile) {
@@ -1009,6 +1022,7 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
 // Inputs of coupling_particle loaded before the staging, so that its round trips to memory cover
 // theirs.
 struct CouplingInputs : Staged {
+  static constexpr bool kStages = true;
   static constexpr int kBatch = 3;
   float xs[3], vs[3], ms, vl;
   uint32_t fl;

@@ -142,7 +142,8 @@ class LBMMpmCoupler:
             nat.call("fsi_coupled_substep", *common, nat.ptr(mpm.workspace),
                      mpm.workspace.numel(), nat.stream_ptr())
         else:
-            nat.call("fsi_coupled_substep_tiled", *common, nat.ptr(mpm._dirty), nat.stream_ptr())
+            nat.call("fsi_coupled_substep_tiled_storage", self.lbm._desc.storage, *common,
+                     nat.ptr(mpm._dirty), nat.stream_ptr())
 
     def _contact_kernel(self) -> None:
         nat.call("fsi_contact", self._desc, self.mpm.desc, self.mpm.particles,
