@@ -32,7 +32,7 @@ __device__ __forceinline__ void stencil_base(float inv_dx, const float x[3], int
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float g = __fmul_rn(x[a], inv_dx);
-    base[a] = (int)__fsub_rn(g, 0.5f);
+    base[a] = base_cell(__fsub_rn(g, 0.5f));
     fx[a] = __fsub_rn(g, (float)base[a]);
   }
 }
@@ -118,8 +118,7 @@ __device__ __forceinline__ bool coupling_particle(const ForceArgs& a, int p, int
   valid = 0.f;
   float uf[3] = {0.f, 0.f, 0.f};
   usable = 0;
-  const bool interior = base[0] >= 0 && base[0] + 2 < a.g.nx && base[1] >= 0 &&
-                        base[1] + 2 < a.g.ny && base[2] >= 0 && base[2] + 2 < a.g.nz;
+  const bool interior = stencil_inside(a.g, base);
   if (interior) {
     // The whole stencil lies in the lattice: the flag word of its centre node says which of
     // the 27 nodes are fluid, so the lattice-velocity loads go out together (an x-plane of 9
@@ -359,8 +358,7 @@ __device__ __forceinline__ void coupling_spread_body(const ForceArgs& a, int p) 
     for (int i = 0; i < 3; ++i) wv[ax][i] = bspline_w(fx[ax], i);
   uint32_t usable = 0;
   const long long sx = (long long)a.g.ny * a.g.nz, sy = a.g.nz;
-  if (base[0] >= 0 && base[0] + 2 < a.g.nx && base[1] >= 0 && base[1] + 2 < a.g.ny &&
-      base[2] >= 0 && base[2] + 2 < a.g.nz) {
+  if (stencil_inside(a.g, base)) {
     const uint32_t fl = a.flags[(base[0] + 1) * sx + (base[1] + 1) * sy + (base[2] + 1)];
 #pragma unroll
     for (int s = 0; s < 27; ++s) usable |= ((~fl >> stencil_flag_bit(s)) & 1u) << s;

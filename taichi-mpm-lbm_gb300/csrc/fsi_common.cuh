@@ -67,6 +67,17 @@ __host__ __device__ constexpr int ez(int q) {
 // Threads per block of the one-thread-per-item kernels.
 constexpr int kBlock = 256;
 
+// Base cell of a grid coordinate less 1/2 (cast toward zero). The cast saturates at the largest int;
+// kept below it so that base + 2 does not overflow and a stencil far outside stays outside.
+__device__ __forceinline__ int base_cell(float c) { return min((int)c, 0x7fffffff - 2); }
+
+// Whether the stencil of base cell `base` lies in the grid.
+template <class G>
+__device__ __forceinline__ bool stencil_inside(const G& g, const int base[3]) {
+  return base[0] >= 0 && base[0] + 2 < g.nx && base[1] >= 0 && base[1] + 2 < g.ny && base[2] >= 0 &&
+         base[2] + 2 < g.nz;
+}
+
 // Quadratic B-spline weight of offset i (mpm3d.py:227-232).
 __device__ __forceinline__ float bspline_w(float fx, int i) {
   if (i == 0) { float a = __fsub_rn(1.5f, fx); return __fmul_rn(0.5f, __fmul_rn(a, a)); }

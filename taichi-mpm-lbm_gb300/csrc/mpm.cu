@@ -161,10 +161,8 @@ __global__ void base_cells_kernel(Mpm m, PView P, int32_t* __restrict__ out) {
   if (p >= m.n) return;
   float x[3];
   load_particle_x(P, m.cap, p, x);
-  int base[3];
-  float fx[3];
-  base_fx(m, x, base, fx);
-  out[3 * p] = base[0]; out[3 * p + 1] = base[1]; out[3 * p + 2] = base[2];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) out[3 * p + a] = (int)__fsub_rn(__fmul_rn(x[a], m.inv_dx), 0.5f);
 }
 
 __device__ __forceinline__ double wsum(double v) {

@@ -45,7 +45,7 @@ __device__ __forceinline__ void base_fx(const Mpm& m, const float x[3], int base
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float gpos = __fmul_rn(x[a], m.inv_dx);
-    base[a] = (int)__fsub_rn(gpos, 0.5f);
+    base[a] = base_cell(__fsub_rn(gpos, 0.5f));
     fx[a] = __fsub_rn(gpos, (float)base[a]);
   }
 }
@@ -998,8 +998,7 @@ __device__ __forceinline__ void g2p_body(const Mpm& m, const PView& P,
   if (!act) return;
   if (st.ok) {
     auto staged = [&](int i, int j, const bool*) { return [&st, i, j](int k, float v[3]) { st(i, j, k, v); }; };
-    if (base[0] >= 0 && base[0] + 2 < m.nx && base[1] >= 0 && base[1] + 2 < m.ny && base[2] >= 0 &&
-        base[2] + 2 < m.nz)
+    if (stencil_inside(m, base))
       g2p_gather<true>(m, P, p, base, fx, staged);
     else
       g2p_gather<false>(m, P, p, base, fx, staged);
@@ -1058,8 +1057,7 @@ __device__ __forceinline__ void coupling_staged_body(const ForceArgs& a, int p, 
   float fx[3];
   if (act) stencil_base(a.c.inv_dx, in.xs, base, fx);
   in.fl = 0;
-  if (act && base[0] >= 0 && base[0] + 2 < a.g.nx && base[1] >= 0 && base[1] + 2 < a.g.ny && base[2] >= 0 &&
-      base[2] + 2 < a.g.nz)
+  if (act && stencil_inside(a.g, base))
     in.fl = a.flags[((long long)(base[0] + 1) * a.g.ny + base[1] + 1) * a.g.nz + base[2] + 1];
   static_cast<Staged&>(in) =
       stage_stencils(a.g, act, base, tile, scratch, [&](int i, int j, int k, float v[3]) {
