@@ -38,16 +38,13 @@ inline unsigned grid_for(long long n, int block) {
   return (unsigned)(g < 1 ? 1 : g);
 }
 
-// Opts kernel K into `bytes` of dynamic shared memory, once per device.
+// Opts kernel K into `bytes` of dynamic shared memory. On every launch that needs it: the attribute
+// belongs to the kernel in the current context, which a host may reset or exchange for another.
 template <auto K>
 int opt_in_smem(int bytes) {
-  static bool done[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return check_launch("cudaGetDevice");
-  if (dev >= 0 && dev < 64 && done[dev]) return FSI_OK;
-  if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+  if (bytes > 48 * 1024 &&
+      cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
     return check_launch("cudaFuncSetAttribute(shared memory)");
-  if (dev >= 0 && dev < 64) done[dev] = true;
   return FSI_OK;
 }
 
