@@ -546,12 +546,25 @@ class ClosureTrainer:
         self.rows_t.clear()
         return int(self.x.shape[0])
 
+    def _check_rows(self) -> None:
+        """The data set is read by row number on the device, without a bound there."""
+        x, t, dev = self.x, self.t, self.net.params.device
+        if x.ndim != 2 or x.shape[1] != FEATURES or x.dtype != torch.bfloat16 or x.shape[0] == 0:
+            raise ValueError(f"feature rows must be bfloat16 [n, {FEATURES}], n > 0; got "
+                             f"{x.dtype} {list(x.shape)}.")
+        if t.ndim != 2 or t.shape[1] != OUT or t.dtype != torch.float32 or t.shape[0] < x.shape[0]:
+            raise ValueError(f"targets must be float32 [n, {OUT}] for the {x.shape[0]} feature rows; "
+                             f"got {t.dtype} {list(t.shape)}.")
+        if x.device != dev or t.device != dev:
+            raise ValueError(f"rows on {x.device} and {t.device}, the network on {dev}.")
+
     def fit(self, steps: int = 500, batch: int = 16384, lr: float = 2e-3, seed: int = 0,
             halvings: float = 3.0) -> list[float]:
         """Adam on random mini-batches (multiples of 128 rows), the learning rate halving
         ``halvings`` times over the run; returns the loss history. Each step is one call
         (``fsi_closure_train_step``): the passes of ``ClosureMLP.forward`` / ``backward`` /
         ``adam_step`` with the rows picked on the device."""
+        self._check_rows()
         g = torch.Generator(device="cpu").manual_seed(seed)
         n = self.x.shape[0]
         batch = max(128, min(batch, n) // 128 * 128)
