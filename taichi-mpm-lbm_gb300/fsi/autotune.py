@@ -6,13 +6,13 @@ Batched step: candidates are (cells per thread block, register-cap variant) pair
 Each is timed with CUDA events over a few lattice steps of the actual batch, from a
 snapshot of the batch's state that is restored afterwards, so tuning leaves the
 simulation where it was. The fastest choice is applied and stored, with every candidate's
-timing, in a JSON cache keyed by the GPU, the storage / arithmetic form and the batch's
-lattice sizes, so a later batch of the same shape starts tuned.
+timing, in a JSON cache keyed by the GPU, ``LAUNCH_SET``, the storage / arithmetic form and the
+batch's lattice sizes, so a later batch of the same shape starts tuned.
 
 Coupled substep: candidates are (threads per block of P2G and G2P, coupling placement) pairs
 of the tiled scatter's descriptor fields (``fsi_mpm_desc.launch_threads``, ``coupling_fold``),
 timed on whole coupled steps of the simulation from a snapshot of its state that is restored
-afterwards, cached under the GPU, grid shape, particle count, scatter mode and storage.
+afterwards, cached under the GPU, ``LAUNCH_SET``, grid shape, particle count, scatter mode and storage.
 """
 from __future__ import annotations
 
@@ -26,6 +26,11 @@ import torch
 from . import _native as nat
 
 
+# What the tuned numbers stand for. Raised whenever a register-cap variant, a block size or a coupling
+# placement comes to mean another kernel, so that records of the kernels before it are not applied.
+LAUNCH_SET = 2
+
+
 def cache_path() -> Path:
     return Path(os.environ.get("FSI_AUTOTUNE_CACHE",
                                Path.home() / ".cache" / "fsi_gb300" / "autotune.json"))
@@ -34,7 +39,7 @@ def cache_path() -> Path:
 def _signature(batch) -> str:
     c0 = batch.configs[0]
     shapes = sorted(batch.shapes)
-    text = json.dumps([torch.cuda.get_device_name(), c0.population_storage,
+    text = json.dumps([torch.cuda.get_device_name(), LAUNCH_SET, c0.population_storage,
                        c0.resolved_arithmetic(), shapes])
     return hashlib.sha1(text.encode()).hexdigest()
 
@@ -112,7 +117,7 @@ def coupled_signature(sim) -> str:
     n = max(int(sim.mpm.particle_count()), 1)
     bucket = 1 << max(n.bit_length() - 5, 0)
     c = sim.config
-    text = json.dumps([torch.cuda.get_device_name(), "coupled", [c.lbm.nx, c.lbm.ny, c.lbm.nz],
+    text = json.dumps([torch.cuda.get_device_name(), LAUNCH_SET, "coupled", [c.lbm.nx, c.lbm.ny, c.lbm.nz],
                        (n + bucket - 1) // bucket * bucket, c.mpm.p2g_mode,
                        c.lbm.population_storage])
     return hashlib.sha1(text.encode()).hexdigest()
