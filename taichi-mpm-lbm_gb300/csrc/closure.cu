@@ -1435,7 +1435,9 @@ constexpr int kOffB1 = kH * kK1, kOffW2p = kOffB1 + kH, kOffB2 = kOffW2p + kH * 
               kOffW3p = kOffB2 + kH, kOffB3 = kOffW3p + kH * kH, kOffW4p = kOffB3 + kH,
               kOffB4 = kOffW4p + kOutPad * kH, kParams = kOffB4 + kOutPad;
 
-// Rows per block of a split weight gradient: 64 blocks of 256 rows for 16,384 rows.
+// Rows per block of a split weight gradient, chosen for batches of 16,384 rows: 64 blocks a hidden
+// layer, 32 x 6 for W1 with twice as many rows. Smaller batches launch fewer blocks (1,024 rows: 4
+// and 2 x 6).
 constexpr int kTrainChunk = 256;
 
 struct NetCopies {
@@ -1588,7 +1590,7 @@ extern "C" int fsi_closure_train_step(const fsi_closure_train_desc* d, void* str
                    nullptr, w.z[1])) return e;
   if (int e = gemm(w.dz[1], d->w2t, kH, m, kH, kH, kGeluBwd, kH, nullptr, 0, nullptr, w.dz[0], w.dzt[0],
                    nullptr, w.z[0])) return e;
-  // weight gradients: split over the rows so that every SM has a block or two
+  // weight gradients: split over the rows (kTrainChunk)
   const int chunk = kTrainChunk;
   if (int e = gemm(w.dyt, w.ht[2], m, kOutPad, kH, m, kAtomicF32, chunk, gr + kOffW4p, kH, nullptr, nullptr,
                    nullptr, nullptr, nullptr)) return e;

@@ -538,7 +538,6 @@ __global__ void __launch_bounds__(kStepBlock, (step_min_blocks<kStore, kFast, kO
   step_cells<kStore, kFast, kOdd, kRecompute, StepArgs>(a, ci, cj, ck, has);
 }
 
-// numpy float32 norm of a 3-vector: sqrt((x*x + y*y) + z*z).
 // Minimum resident blocks per SM of the even step by pairs. us per step at 256^3 with rho and u
 // read / recomputed, by blocks: FP16 331/322 at 5, 334/316 at 6, 312/314 at 7, 312/322 at 8; BF16
 // 318/316, 291/308, 284/317, 294/316; fast FP32 430/405, 428/423, 430/419, 446/497.
@@ -607,6 +606,7 @@ __global__ void __launch_bounds__(kStepBlock, (even_min_blocks<kStore, kRecomput
   if (c < (uint32_t)a.g.n) step_even_pair<kStore, kRecompute>(a, c);
 }
 
+// numpy float32 norm of a 3-vector: sqrt((x*x + y*y) + z*z).
 __device__ __forceinline__ float norm3_ref(float x, float y, float z) {
   return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)));
 }

@@ -10,13 +10,14 @@
 //             Touched 4^3 node blocks are marked dirty. The coupled substep forms
 //             each particle's penalty force in a separate kernel before it, or on
 //             small launches in the same pass, which then scatters through a
-//             shared-memory tile of nodes.
+//             shared-memory tile of nodes, as do the launches beside 16-bit lattices.
 //   2. g2p:   grid update (p/m + dt g, sticky/damped walls) fused into the
 //             gather: a CTA stages the grid-updated velocities of its stencil box
 //             (two boxes where it ends one body and begins the next) in shared
 //             memory, then each particle gathers v and the APIC C, advects and clamps.
 //   3. clear: zeroes the dirty blocks, restoring the all-zero grid.
-// Arithmetic follows the reference's float32 operation order (no contraction).
+// Arithmetic follows the reference's float32 operation order (no contraction), but for P2G in
+// runs, whose terms and sums are fused multiply-adds in float32.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -30,8 +31,8 @@ namespace {
 // P2G is capped at 64 registers (32 warps per SM, against 24 at its natural 75-80): the extra
 // resident warps hide more of the latency of its phases; G2P at 48 (40 warps): 2,097,152 particles
 // gather in 109 us, against 117 at 64 registers (no spills) and 133 at its natural 72.
-// Threads per P2G / G2P block kT (m.threads): 128, 256 or 512, each at the same cap; P2G's shared
-// memory is dynamic.
+// Threads per P2G / G2P block kT (m.threads): 128, 256 or 512, each at the same cap, but for G2P of
+// 512 threads, of which two blocks fit (64 registers). P2G's shared memory is dynamic.
 template <int kT>
 __global__ void __launch_bounds__(kT, 1024 / kT) p2g_kernel(Mpm m, PView P,
                                                             float4* __restrict__ grid,
