@@ -54,12 +54,20 @@ def _substep(where, storage, pos, set_state):
         m.initialize_particles_from_numpy(p)
         set_state(i, *(t[..., :len(p)] for t in (m._x, m._v, m._C, m._F, m._mass)))
         m.desc.coupling_fold = 2  # the kernels of large launches
-        LBMMpmCoupler(coupling, s, m)._coupled_substep(0.1, 0.1, False)
+        c = LBMMpmCoupler(coupling, s, m)
+        if where == "single":
+            c._coupled_substep(0.1, 0.1, False)
+        else:  # the entry point that does not know the lattice's storage
+            c._desc.gamma_eff, c._desc.dt_ratio, c._desc.build_fraction = 0.0, 0.1, 0
+            m.desc.dt = 0.1
+            nat.call("fsi_coupled_substep_tiled", c._desc, m.desc, m.particles, nat.ptr(s.macro), nat.ptr(s.flags),
+                     nat.ptr(c._accum), nat.ptr(c._valid), nat.ptr(c._mask), nat.ptr(c._counters),
+                     nat.ptr(m._grid), nat.ptr(m._dirty), nat.stream_ptr())
         out.append([t[..., :len(p)].cpu().numpy().T for t in (m._x, m._v, m._C, m._F)])
     return out
 
 
-@pytest.mark.parametrize("where", ["batch", "single"])
+@pytest.mark.parametrize("where", ["batch", "single", "untold"])
 @pytest.mark.parametrize("storage", ["f16", "bf16"])
 def test_terms_are_rounded_one_by_one(where, storage):
     rng = np.random.default_rng(7)
@@ -84,7 +92,7 @@ def test_terms_are_rounded_one_by_one(where, storage):
             np.testing.assert_array_equal(g, np.asarray(w[:len(p)]).reshape(g.shape))
 
 
-@pytest.mark.parametrize("where", ["batch", "single"])
+@pytest.mark.parametrize("where", ["batch", "single", "untold"])
 @pytest.mark.parametrize("storage", ["f16", "bf16"])
 def test_a_block_adds_to_a_node_once(where, storage):
     spots = [(5.5, 6.5, 7.5), (20.5, 21.5, 9.5), (12.5, 5.5, 25.5), (25.5, 25.5, 25.5)]
